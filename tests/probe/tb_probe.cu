@@ -36,6 +36,8 @@ __global__ void k_probe_math(const double* __restrict__ x, int64_t n, int fn, do
     case 0: r = rcp_nr(v); break;
     case 1: r = rsqrt_nr(v); break;
     case 2: r = log_bf(v); break;
+    case 3: r = rsqrt_h3(v); break;
+    case 4: r = neglog_tab(v); break;
     case 10: r = 1.0 / v; break;
     case 11: r = 1.0 / sqrt(v); break;
     default: r = log(v); break;

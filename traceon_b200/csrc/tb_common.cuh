@@ -215,6 +215,14 @@ __device__ __forceinline__ double ring_pot_nopi(double r0, double z0, double rs,
 // Accumulates one weighted ring into the partial field sums.  After the
 // whole reduction, E_r = Sr / (2 pi r0) (0 on the axis) and E_z = -Sz / pi.
 // Optionally accumulates the potential sum Sp (phi = Sp / pi).
+//
+// The sums are bound by the FP64 pipe, so what counts is the number of FP64
+// instructions per pair.  One reciprocal square root serves both 1 / sqrt(D)
+// and 1 / rho2: g = 1 / (rho2 sqrt(D)) = rsqrt(rho2^2 D), 1 / sqrt(D) =
+// rho2 g; and the logarithm comes from a table (tb_fastmath.cuh).  Measured
+// against separate reciprocals with two Newton steps each and a series
+// logarithm (same direct sums): 2^18 points x 262,144 rings 563 -> 410 ms,
+// 4,096 electrons through 16,000 rings 240 -> 195 ms; differences 1e-16.
 template <bool WANT_POT>
 __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, double zs, double w,
                                                double& Sr, double& Sz, double& Sp) {
@@ -223,15 +231,15 @@ __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, 
   double rho2 = fma(dr, dr, dz2);
   double s = rs + r0;
   double D = fma(s, s, dz2);
-  double ir = rcp_nr(rho2);        // 1 / rho2
-  double rD = rsqrt_nr(D);         // 1 / sqrt(D)
+  double g = rsqrt_h3(rho2 * rho2 * D);
+  double rD = rho2 * g;            // 1 / sqrt(D)
   double t = rho2 * rD * rD;       // rho2 / D
   double t2 = t * t, t4 = t2 * t2;
-  double L = -log_bf(t);
+  double L = neglog_tab(t);
   double K = fma(L, estrin8(C_KB, t, t2, t4), estrin8(C_KA, t, t2, t4));
   double E = fma(L, estrin8(C_EB, t, t2, t4), estrin8(C_EA, t, t2, t4));
-  double c = w * rs * rD * ir;     // w rs / (rho2 sqrt(D))
-  double m = fma(dr, dr - 2.0 * rs, -dz2);   // dr^2 - 2 dr rs - dz^2
+  double c = w * rs * g;           // w rs / (rho2 sqrt(D))
+  double m = fma(dr, fma(-2.0, rs, dr), -dz2);   // dr^2 - 2 dr rs - dz^2
   Sr = fma(c, fma(rho2, K, m * E), Sr);
   Sz = fma(c * dz, E, Sz);
   if (WANT_POT) Sp = fma(c * rho2, K, Sp);
