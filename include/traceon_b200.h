@@ -414,6 +414,18 @@ int tb_current_axial_derivatives(const double *z, int64_t Nz, const double *sour
 int tb_field_radial_points(const double *points, int64_t M, const double *sources, int64_t Nq, double *pot,
                            double *field, tb_stream_t stream);
 
+/* The same through a tree of the rings: the rings of every straight,
+ * axis-parallel stretch are gathered into 16 proxy rings per range of
+ * elements, and a point sums the proxies of the ranges that are far enough
+ * from it and the rings of the others.  The sums agree with the direct ones to
+ * the accuracy of the ring kernels.  `sources` in the order of
+ * tb_pack_sources (16 rings per element).  work (16-byte aligned):
+ * tb_field_points_workspace(M, Nq) bytes; where that is 0 (few pairs, or rings
+ * that are not whole elements) or work is NULL, the direct sums run. */
+int64_t tb_field_points_workspace(int64_t M, int64_t Nq);
+int tb_field_radial_points_ws(const double *points, int64_t M, const double *sources, int64_t Nq, double *pot,
+                              double *field, void *work, int64_t work_bytes, tb_stream_t stream);
+
 /* Axial derivatives at N_z points, radial.c:18-36 (overwrites derivs
  * (N_z, 9)). */
 int tb_axial_derivatives_radial(const double *z, int64_t Nz, const double *sources, int64_t Nq,
@@ -486,6 +498,20 @@ int tb_trace_rk45_geometries(const double *start, const double *t0, const double
                              const double *geom_bounds, const tb_trace_opts_t *opts, double *rows, int64_t *nrows, int32_t *status,
                              double *final_state, double *plane, int64_t *counters, int32_t *work,
                              tb_stream_t stream);
+
+/* tb_trace_rk45 (geom NULL) and tb_trace_rk45_geometries through a tree of the
+ * electrostatic rings, as tb_field_radial_points_ws: every call builds it in
+ * tree_work (16-byte aligned) before it traces.  Fields with magnetostatic or
+ * current rings are summed directly.
+ * tb_trace_workspace gives the bytes (n_geoms: 0 without geom); where that is
+ * 0 or tree_work is NULL, the direct sums run.  With geom the source offsets
+ * have to be multiples of 16. */
+int64_t tb_trace_workspace(const tb_field_t *field, int64_t n, int64_t n_geoms);
+int tb_trace_rk45_ws(const double *start, const double *t0, const double *qm, const int32_t *geom, int64_t n,
+                     const tb_field_t *field, const int64_t *src_offsets, int64_t n_geoms, const double *geom_bounds,
+                     const tb_trace_opts_t *opts, double *rows, int64_t *nrows, int32_t *status, double *final_state,
+                     double *plane, int64_t *counters, int32_t *work, void *tree_work, int64_t tree_bytes,
+                     tb_stream_t stream);
 
 /* Plane crossings of trajectories stored by tb_trace_rk45 (device arrays):
  * per trajectory the crossing nearest its end, by linear interpolation, as

@@ -217,6 +217,7 @@ _DEV = {
     'tb_pack_sources': (vp, vp, vp, vp, i64, vp),
     'tb_pack_current_sources': (vp, vp, vp, vp, i64, vp),
     'tb_field_radial_points': (vp, i64, vp, i64, vp, vp, vp),
+    'tb_field_radial_points_ws': (vp, i64, vp, i64, vp, vp, vp, i64, vp),
     'tb_current_field_points': (vp, i64, vp, i64, vp, vp),
     'tb_axial_derivatives_radial': (vp, i64, vp, i64, vp, vp),
     'tb_current_axial_derivatives': (vp, i64, vp, i64, vp, vp),
@@ -225,6 +226,8 @@ _DEV = {
     'tb_trace_rk45': (vp, vp, vp, i64, C.POINTER(TbField), C.POINTER(TbTraceOpts), vp, vp, vp, vp, vp, vp, vp, vp),
     'tb_trace_rk45_geometries': (vp, vp, vp, vp, i64, C.POINTER(TbField), vp, i64, vp, C.POINTER(TbTraceOpts), vp, vp,
                                  vp, vp, vp, vp, vp, vp),
+    'tb_trace_rk45_ws': (vp, vp, vp, vp, i64, C.POINTER(TbField), vp, i64, vp, C.POINTER(TbTraceOpts), vp, vp, vp, vp,
+                         vp, vp, vp, vp, i64, vp),
     'tb_batch_solve': (vp, C.c_int, vp, i64, vp, vp, i64, vp, i64, vp, C.c_int, vp),
     'tb_num_sms': (),
     'tb_lu_nopiv_f64': (vp, i64, i64, vp),
@@ -241,6 +244,10 @@ for _name, _args in _DEV.items():
     _f = getattr(backend_lib, _name)
     _f.restype = C.c_int
     _f.argtypes = list(_args)
+backend_lib.tb_field_points_workspace.restype = i64
+backend_lib.tb_field_points_workspace.argtypes = [i64, i64]
+backend_lib.tb_trace_workspace.restype = i64
+backend_lib.tb_trace_workspace.argtypes = [C.POINTER(TbField), i64, i64]
 backend_lib.tb_batch_solve_plan.restype = i64
 backend_lib.tb_batch_solve_plan.argtypes = [vp, C.c_int, vp, C.POINTER(i64)]
 backend_lib.tb_set_solve_lookahead.restype = C.c_int
@@ -581,6 +588,22 @@ def to_dev(a, dtype=None):
     return torch.as_tensor(np.ascontiguousarray(a), device=device(), dtype=dtype).contiguous()
 
 
+def dev_scratch(nbytes, device, stream=None):
+    """Device scratch (uint8) for a call on `stream` (a raw stream, default the
+    current one), or None for 0 bytes and when memory is short: every call that
+    takes such scratch has a form without."""
+    torch = _torch()
+    if nbytes <= 0:
+        return None
+    try:
+        t = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    except torch.OutOfMemoryError:
+        return None
+    if stream is not None and stream != _stream():  # used there, allocated here
+        t.record_stream(torch.cuda.ExternalStream(stream, device=device))
+    return t
+
+
 def dev_jacobian_buffer(vertices_t):
     torch = _torch()
     N = vertices_t.shape[0]
@@ -796,8 +819,11 @@ def dev_field_points(points_t, sources_t, want_pot=True, want_field=True):
     pot = torch.empty(M, dtype=torch.float64, device=points_t.device) if want_pot else None
     field = torch.empty((M, 3), dtype=torch.float64, device=points_t.device) if want_field else None
     if M:
-        _call('tb_field_radial_points', _ptr(points_t), M, _ptr(sources_t), sources_t.shape[1], _ptr(pot),
-              _ptr(field), _stream())
+        Nq = sources_t.shape[1]
+        nbytes = backend_lib.tb_field_points_workspace(M, Nq)
+        work = dev_scratch(nbytes, points_t.device)
+        _call('tb_field_radial_points_ws', _ptr(points_t), M, _ptr(sources_t), Nq, _ptr(pot), _ptr(field), _ptr(work),
+              nbytes, _stream())
     return pot, field
 
 

@@ -1,7 +1,7 @@
 """The batching workload's device pipeline: many geometries of uneven N
 filled, factored and solved in ONE persistent launch (tb_batch_solve), then
 all their particles traced through the direct BEM field in one more
-(tb_trace_rk45_geometries), the two captured as one CUDA graph.
+(tb_trace_rk45_ws), the two captured as one CUDA graph.
 
 The reference fills and solves one excitation at a time
 (traceon/solver.py:160-232, 402-431) and traces one field at a time
@@ -117,7 +117,7 @@ class BatchSolve:
 
 class BatchPipeline:
     """fill -> factor -> solve -> pack (tb_batch_solve) -> trace
-    (tb_trace_rk45_geometries) for many geometries, enqueued together and,
+    (tb_trace_rk45_ws) for many geometries, enqueued together and,
     with capture(), recorded as one CUDA graph that replay() re-runs.
     positions[g], velocities[g]: (n_g, 3) start states of geometry g's
     particles; bounds[g]: its (3, 2) box.  Particles' end states (t, x, y, z,
@@ -154,14 +154,17 @@ class BatchPipeline:
         o.max_attempts, o.max_rows, o.team_warps = int(max_attempts), 0, int(team_warps)
         self.opts = o
         self.graph = None
+        self.tree_bytes = B.backend_lib.tb_trace_workspace(C.byref(self.field), n, G)
+        self.tree = B.dev_scratch(self.tree_bytes, dev)
 
     def enqueue(self):
         """The two launches on the current stream."""
         self.batch.launch()
-        B._call('tb_trace_rk45_geometries', self.start.data_ptr(), None, self.qm.data_ptr(), self.geom.data_ptr(),
+        B._call('tb_trace_rk45_ws', self.start.data_ptr(), None, self.qm.data_ptr(), self.geom.data_ptr(),
                 self.n, C.byref(self.field), self.batch.ring_offsets.data_ptr(), len(self.batch),
                 self.gbounds.data_ptr(), C.byref(self.opts), None, None, self.status.data_ptr(),
-                self.final.data_ptr(), None, self.counters.data_ptr(), self.work.data_ptr(), B._stream())
+                self.final.data_ptr(), None, self.counters.data_ptr(), self.work.data_ptr(), B._ptr(self.tree),
+                self.tree_bytes, B._stream())
 
     def trace_subset(self, idx, team_warps: int, max_attempts: int = 2000):
         """The trace launch on the particles idx (a device index tensor) with
@@ -179,10 +182,11 @@ class BatchPipeline:
         o = B.TbTraceOpts.from_buffer_copy(self.opts)
         o.team_warps = int(team_warps)
         o.max_attempts = min(int(o.max_attempts), int(max_attempts))
-        B._call('tb_trace_rk45_geometries', st.data_ptr(), None, qm.data_ptr(), geom.data_ptr(), m,
+        tree = B.dev_scratch(self.tree_bytes, st.device)
+        B._call('tb_trace_rk45_ws', st.data_ptr(), None, qm.data_ptr(), geom.data_ptr(), m,
                 C.byref(self.field), self.batch.ring_offsets.data_ptr(), len(self.batch), self.gbounds.data_ptr(),
                 C.byref(o), None, None, status.data_ptr(), final.data_ptr(), None, counters.data_ptr(),
-                work.data_ptr(), B._stream())
+                work.data_ptr(), B._ptr(tree), self.tree_bytes, B._stream())
         return final
 
     def capture(self):

@@ -269,23 +269,6 @@ __device__ __forceinline__ void source_sums(double r0, double z0, const double* 
   for (int64_t j = first; j < Nq; j += stride) ring_field_acc<POT>(r0, z0, sr[j], sz[j], sw[j], Sr, Sz, Sp);
 }
 
-__device__ __forceinline__ void finish_field(const double* p, double Sr, double Sz, double Sp, double* pot,
-                                             double* field, int64_t m) {
-  double r = sqrt(p[0] * p[0] + p[1] * p[1]);
-  if (pot) pot[m] = Sp * INV_PI;
-  if (field) {
-    double Er = r >= MIN_AXIS ? Sr / (2 * PI * r) : 0.0;
-    if (r >= MIN_AXIS) {
-      field[3 * m] = p[0] / r * Er;
-      field[3 * m + 1] = p[1] / r * Er;
-    } else {
-      field[3 * m] = 0.0;
-      field[3 * m + 1] = 0.0;
-    }
-    field[3 * m + 2] = -Sz * INV_PI;
-  }
-}
-
 // One thread per point; source tiles staged through shared memory.
 constexpr int FP_THREADS = 256;
 template <bool POT>
@@ -300,7 +283,7 @@ __global__ void __launch_bounds__(FP_THREADS)
     p[1] = points[3 * m + 1];
     p[2] = points[3 * m + 2];
   }
-  double r0 = sqrt(p[0] * p[0] + p[1] * p[1]), z0 = p[2];
+  double r0 = axis_distance(p), z0 = p[2];
   double Sr = 0, Sz = 0, Sp = 0;
   for (int64_t base = 0; base < Nq; base += FP_THREADS) {
     int64_t j = base + threadIdx.x;
@@ -336,7 +319,7 @@ __global__ void __launch_bounds__(TEAM >= 256 ? TEAM : 256)
     p[1] = points[3 * m + 1];
     p[2] = points[3 * m + 2];
   }
-  double r0 = sqrt(p[0] * p[0] + p[1] * p[1]);
+  double r0 = axis_distance(p);
   double Sr = 0, Sz = 0, Sp = 0;
   if (m < M) source_sums<POT>(r0, p[2], src, Nq, lane, TEAM, Sr, Sz, Sp);
   Sr = warp_sum(Sr);
@@ -514,7 +497,7 @@ __global__ void k_current_field_points(const double* __restrict__ points, int64_
   int lane = threadIdx.x & 31;
   if (m >= M) return;
   double p[3] = {points[3 * m], points[3 * m + 1], points[3 * m + 2]};
-  double r = sqrt(p[0] * p[0] + p[1] * p[1]);
+  double r = axis_distance(p);
   double Br = 0, Bz = 0;
   for (int64_t j = lane; j < Nc; j += 32) {
     double hr, hz;

@@ -69,6 +69,13 @@ __constant__ double C_EB[8] = {0.0, 2.49999998448655e-1, 9.37488062098189e-2, 5.
                                4.09074821593164e-2, 2.35091602564984e-2, 6.45682247315060e-3,
                                3.78886487349367e-4};
 
+// G(1-p) = C + D with D = (K - E) / m, B = K - D, C = (D - B) / m, m = 1 - p:
+// the same log-polynomial form, degree 8, fitted by weighted minimax (Lawson's
+// iteration in 50-digit arithmetic) to 5e-14 of G / sqrt(p); the ring field's
+// radial part (ring_field_acc) multiplies it by p.
+__constant__ double C_GA[9] = {-0.22741127658373964, -0.5911141960607428, -0.6197405483508255, -0.6023516855041392, -0.29322383698435994, 0.845529509167207, 1.6550608315837363, 0.7513620739234596, 0.06363683305616191};
+__constant__ double C_GB[9] = {0.9999999998835012, 1.4999995930911356, 2.109254695511045, 2.726924230368857, 3.2243731023450963, 3.0145646707960214, 1.6279693370132986, 0.34046951681463455, 0.014327341145446069};
+
 __device__ __forceinline__ double horner_c(const double* c, double p) {
   double s = c[7];
 #pragma unroll
@@ -212,9 +219,18 @@ __device__ __forceinline__ double ring_pot_nopi(double r0, double z0, double rs,
   return K * rs * rD;
 }
 
+// The same for degree 8.
+__device__ __forceinline__ double estrin9(const double* c, double t, double t2, double t4) {
+  double a = fma(c[1], t, c[0]);
+  double b = fma(c[3], t, c[2]);
+  double d = fma(c[5], t, c[4]);
+  double e = fma(fma(c[8], t, c[7]), t, c[6]);
+  return fma(t4, fma(t2, e, d), fma(t2, b, a));
+}
+
 // Accumulates one weighted ring into the partial field sums.  After the
-// whole reduction, E_r = Sr / (2 pi r0) (0 on the axis) and E_z = -Sz / pi.
-// Optionally accumulates the potential sum Sp (phi = Sp / pi).
+// whole reduction, E_r = r0 Sr / pi and E_z = -Sz / pi.  Optionally
+// accumulates the potential sum Sp (phi = Sp / pi).
 //
 // The sums are bound by the FP64 pipe, so what counts is the number of FP64
 // instructions per pair.  One reciprocal square root serves both 1 / sqrt(D)
@@ -223,6 +239,16 @@ __device__ __forceinline__ double ring_pot_nopi(double r0, double z0, double rs,
 // against separate reciprocals with two Newton steps each and a series
 // logarithm (same direct sums): 2^18 points x 262,144 rings 563 -> 410 ms,
 // 4,096 electrons through 16,000 rings 240 -> 195 ms; differences 1e-16.
+//
+// Radial part.  -d phi/d r0 as written above, (rho2 K + m E) / r0, is a
+// difference of equal terms near the axis: what K and E are off by (1e-13 at
+// degree 7, 1e-16 by rounding) is multiplied by rs / r0.  With K = B + D,
+// E = B + t D and 2 D - E = m (C + D) = m G, m = 4 r0 rs / D, the factor r0
+// comes out exactly:
+//   E_r = (r0 / pi) sum w rs / (D rho2 sqrt(D)) (4 rs^2 t G + (rho2 - 4 rs dr) E).
+// On the einzel lens, off axis by 0.9, 0.1 and 0.001 mm, the sums' E_r is off
+// by 1.2e-13, 4e-13 and 3e-13 (5.8e-13, 1.4e-11 and 5.5e-9 with K and E), of
+// which rounding is 1e-16 to 1e-15 (9e-16, 2e-14 and 5e-11).
 template <bool WANT_POT>
 __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, double zs, double w,
                                                double& Sr, double& Sz, double& Sp) {
@@ -236,13 +262,39 @@ __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, 
   double t = rho2 * rD * rD;       // rho2 / D
   double t2 = t * t, t4 = t2 * t2;
   double L = neglog_tab(t);
+  double E = fma(L, estrin8(C_EB, t, t2, t4), estrin8(C_EA, t, t2, t4));
+  double G = fma(L, estrin9(C_GB, t, t2, t4), estrin9(C_GA, t, t2, t4));
+  double c = w * rs * g;           // w rs / (rho2 sqrt(D))
+  double q = 4.0 * rs;
+  Sr = fma(c * (rD * rD), fma(q * rs * t, G, fma(-q, dr, rho2) * E), Sr);
+  Sz = fma(c * dz, E, Sz);
+  if (WANT_POT) {
+    double K = fma(L, estrin8(C_KB, t, t2, t4), estrin8(C_KA, t, t2, t4));
+    Sp = fma(c * rho2, K, Sp);
+  }
+}
+
+// The same sums in the form -d phi/d r0 has above, with K and E, separate
+// reciprocals and the series logarithm: E_r = Sr / (2 pi r0), E_z = -Sz / pi.
+// For the BEM tracer's fields with a magnetic part (tb_trace.cu).
+__device__ __forceinline__ void ring_field_acc_ke(double r0, double z0, double rs, double zs, double w, double& Sr,
+                                                  double& Sz) {
+  double dr = rs - r0, dz = zs - z0;
+  double dz2 = dz * dz;
+  double rho2 = fma(dr, dr, dz2);
+  double s = rs + r0;
+  double D = fma(s, s, dz2);
+  double ir = rcp_nr(rho2);        // 1 / rho2
+  double rD = rsqrt_nr(D);         // 1 / sqrt(D)
+  double t = rho2 * rD * rD;       // rho2 / D
+  double t2 = t * t, t4 = t2 * t2;
+  double L = -log_bf(t);
   double K = fma(L, estrin8(C_KB, t, t2, t4), estrin8(C_KA, t, t2, t4));
   double E = fma(L, estrin8(C_EB, t, t2, t4), estrin8(C_EA, t, t2, t4));
-  double c = w * rs * g;           // w rs / (rho2 sqrt(D))
-  double m = fma(dr, fma(-2.0, rs, dr), -dz2);   // dr^2 - 2 dr rs - dz^2
+  double c = w * rs * rD * ir;     // w rs / (rho2 sqrt(D))
+  double m = fma(dr, dr - 2.0 * rs, -dz2);   // dr^2 - 2 dr rs - dz^2
   Sr = fma(c, fma(rho2, K, m * E), Sr);
   Sz = fma(c * dz, E, Sz);
-  if (WANT_POT) Sp = fma(c * rho2, K, Sp);
 }
 
 // Scalar forms with the reference's argument convention (r0, z0, delta_r,

@@ -29,6 +29,23 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// Distance of p from the axis, with its rounding spelled out: a point may be
+// so close to a ring that the last bit of r0 shows in the field, and all sums
+// at one point are to see the same one.
+__device__ __forceinline__ double axis_distance(const double* p) { return sqrt(fma(p[0], p[0], p[1] * p[1])); }
+
+// Potential and field at p from the raw sums of ring_field_acc.
+__device__ __forceinline__ void finish_field(const double* p, double Sr, double Sz, double Sp, double* pot,
+                                             double* field, int64_t m) {
+  if (pot) pot[m] = Sp * INV_PI;
+  if (field) {
+    const double er = axis_distance(p) >= MIN_AXIS ? Sr * INV_PI : 0.0;  // E_r / r
+    field[3 * m] = p[0] * er;
+    field[3 * m + 1] = p[1] * er;
+    field[3 * m + 2] = -Sz * INV_PI;
+  }
+}
+
 // Status of the last kernel launch on this thread.
 inline int launch_status() {
   cudaError_t e = cudaGetLastError();

@@ -4,7 +4,7 @@
 ``trace_multiple``, ``__call__``; traceon/tracing.py:104-245).  Where the
 reference traces particles one after another on one CPU core, every call
 here launches one persistent GPU kernel for all particles
-(``tb_trace_rk45``).  ``trace_endpoints`` is the batched form used for
+(``tb_trace_rk45_ws``).  ``trace_endpoints`` is the batched form used for
 throughput: it returns only the final state and the crossing of an exit
 plane z = const (cubic Hermite interpolation between the two accepted steps
 that bracket it) instead of whole trajectories.
@@ -142,13 +142,16 @@ class Tracer:
         nrows = torch.empty(n, dtype=torch.int64, device=dev) if max_rows else None
         work = torch.empty(1, dtype=torch.int32, device=dev)
         s = B._stream() if stream is None else stream
-        r = B.backend_lib.tb_trace_rk45(start.data_ptr(), None if t0 is None else t0.data_ptr(), qm.data_ptr(), n,
-                                        C.byref(f), C.byref(o), B._ptr(rows), B._ptr(nrows), status.data_ptr(),
-                                        final.data_ptr(), B._ptr(plane), counters.data_ptr(), work.data_ptr(), s)
+        nbytes = B.backend_lib.tb_trace_workspace(C.byref(f), n, 0)
+        tree = B.dev_scratch(nbytes, dev, s)
+        r = B.backend_lib.tb_trace_rk45_ws(start.data_ptr(), None if t0 is None else t0.data_ptr(), qm.data_ptr(),
+                                           None, n, C.byref(f), None, 0, None, C.byref(o), B._ptr(rows),
+                                           B._ptr(nrows), status.data_ptr(), final.data_ptr(), B._ptr(plane),
+                                           counters.data_ptr(), work.data_ptr(), B._ptr(tree), nbytes, s)
         if r != B.TB_OK:
             raise B.BackendError(f'tb_trace_rk45 failed with status {r}')
         res = TraceResult(status, final, plane, counters, rows, nrows)
-        res._keep = (keep, start, qm, t0, work)
+        res._keep = (keep, start, qm, t0, work, tree)
         return res
 
     def _start(self, position, velocity, mass, charge):
@@ -219,7 +222,7 @@ class Tracer:
 def trace_geometries(fields, bounds, positions, velocities, plane_z, mass=m_e, charge=-e, atol=1e-8,
                      max_attempts=DEFAULT_MAX_ATTEMPTS, team_warps=0):
     """Endpoint tracing of particles through several geometries in one GPU
-    launch (tb_trace_rk45_geometries): fields[g] is a FieldRadialBEM
+    launch (tb_trace_rk45_ws): fields[g] is a FieldRadialBEM
     (electrostatic charges only, no field bounds) and positions[g],
     velocities[g] (n_g, 3) its particles.  The reference traces one field at
     a time.  Returns, per geometry, (plane (n_g, 7), final (n_g, 7),
@@ -259,9 +262,11 @@ def trace_geometries(fields, bounds, positions, velocities, plane_z, mass=m_e, c
     plane = torch.empty((n, 7), dtype=torch.float64, device=dev)
     counters = torch.empty((n, 2), dtype=torch.int64, device=dev)
     work = torch.empty(1, dtype=torch.int32, device=dev)
-    B._call('tb_trace_rk45_geometries', start.data_ptr(), None, qm.data_ptr(), geom_t.data_ptr(), n, C.byref(f),
+    nbytes = B.backend_lib.tb_trace_workspace(C.byref(f), n, len(fields))
+    tree = B.dev_scratch(nbytes, dev)
+    B._call('tb_trace_rk45_ws', start.data_ptr(), None, qm.data_ptr(), geom_t.data_ptr(), n, C.byref(f),
             off_t.data_ptr(), len(fields), None, C.byref(o), None, None, status.data_ptr(), final.data_ptr(),
-            plane.data_ptr(), counters.data_ptr(), work.data_ptr(), B._stream())
+            plane.data_ptr(), counters.data_ptr(), work.data_ptr(), B._ptr(tree), nbytes, B._stream())
     out = [a.cpu().numpy() for a in (plane, final, status, counters)]
     cuts = np.cumsum(counts)[:-1]
     return [tuple(x) for x in zip(*(np.split(a, cuts) for a in out))]
