@@ -70,11 +70,10 @@ __constant__ double C_EB[8] = {0.0, 2.49999998448655e-1, 9.37488062098189e-2, 5.
                                3.78886487349367e-4};
 
 // G(1-p) = C + D with D = (K - E) / m, B = K - D, C = (D - B) / m, m = 1 - p:
-// the same log-polynomial form, degree 8, fitted by weighted minimax (Lawson's
-// iteration in 50-digit arithmetic) to 5e-14 of G / sqrt(p); the ring field's
-// radial part (ring_field_acc) multiplies it by p.
-__constant__ double C_GA[9] = {-0.22741127658373964, -0.5911141960607428, -0.6197405483508255, -0.6023516855041392, -0.29322383698435994, 0.845529509167207, 1.6550608315837363, 0.7513620739234596, 0.06363683305616191};
-__constant__ double C_GB[9] = {0.9999999998835012, 1.4999995930911356, 2.109254695511045, 2.726924230368857, 3.2243731023450963, 3.0145646707960214, 1.6279693370132986, 0.34046951681463455, 0.014327341145446069};
+// the same log-polynomial form, degree 9, fitted by minimax (Lawson's
+// iteration in 50-digit arithmetic) to 1e-14 of G.
+__constant__ double C_GA[10] = {-0.2274112777597101, -0.5911168979011567, -0.6203059289734966, -0.6265921919539145, -0.5785563934930864, -0.11125848811773138, 1.208017098098697, 1.784910150068942, 0.692241638383172, 0.05181999589508494};
+__constant__ double C_GB[10] = {0.9999999999999717, 1.4999999977635508, 2.1093725045735865, 2.733973243923425, 3.347779910274752, 3.7576486800388316, 3.255205658767092, 1.5914465500543837, 0.2996988785064158, 0.011424405938099085};
 
 __device__ __forceinline__ double horner_c(const double* c, double p) {
   double s = c[7];
@@ -219,12 +218,12 @@ __device__ __forceinline__ double ring_pot_nopi(double r0, double z0, double rs,
   return K * rs * rD;
 }
 
-// The same for degree 8.
-__device__ __forceinline__ double estrin9(const double* c, double t, double t2, double t4) {
+// The same for degree 9.
+__device__ __forceinline__ double estrin10(const double* c, double t, double t2, double t4) {
   double a = fma(c[1], t, c[0]);
   double b = fma(c[3], t, c[2]);
   double d = fma(c[5], t, c[4]);
-  double e = fma(fma(c[8], t, c[7]), t, c[6]);
+  double e = fma(t2, fma(c[9], t, c[8]), fma(c[7], t, c[6]));
   return fma(t4, fma(t2, e, d), fma(t2, b, a));
 }
 
@@ -247,8 +246,8 @@ __device__ __forceinline__ double estrin9(const double* c, double t, double t2, 
 // comes out exactly:
 //   E_r = (r0 / pi) sum w rs / (D rho2 sqrt(D)) (4 rs^2 t G + (rho2 - 4 rs dr) E).
 // On the einzel lens, off axis by 0.9, 0.1 and 0.001 mm, the sums' E_r is off
-// by 1.2e-13, 4e-13 and 3e-13 (5.8e-13, 1.4e-11 and 5.5e-9 with K and E), of
-// which rounding is 1e-16 to 1e-15 (9e-16, 2e-14 and 5e-11).
+// by 1.1e-13, 3.7e-13 and 2.6e-13 (5.8e-13, 1.4e-11 and 5.5e-9 with K and E), of
+// which rounding is 2e-16 to 4e-16 (9e-16, 2e-14 and 5e-11).
 template <bool WANT_POT>
 __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, double zs, double w,
                                                double& Sr, double& Sz, double& Sp) {
@@ -263,7 +262,7 @@ __device__ __forceinline__ void ring_field_acc(double r0, double z0, double rs, 
   double t2 = t * t, t4 = t2 * t2;
   double L = neglog_tab(t);
   double E = fma(L, estrin8(C_EB, t, t2, t4), estrin8(C_EA, t, t2, t4));
-  double G = fma(L, estrin9(C_GB, t, t2, t4), estrin9(C_GA, t, t2, t4));
+  double G = fma(L, estrin10(C_GB, t, t2, t4), estrin10(C_GA, t, t2, t4));
   double c = w * rs * g;           // w rs / (rho2 sqrt(D))
   double q = 4.0 * rs;
   Sr = fma(c * (rD * rD), fma(q * rs * t, G, fma(-q, dr, rho2) * E), Sr);
