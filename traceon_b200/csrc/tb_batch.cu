@@ -51,6 +51,8 @@ constexpr int LDT = BT + 1; // padded row of a whole tile in shared memory
 constexpr int STAGE_DOUBLES = 2 * BT * KC;
 constexpr int SMEM_DOUBLES = 2 * BT * LDT;  // two tiles (or the GEMM stages)
 static_assert(NSTAGE * STAGE_DOUBLES <= 2 * BT * LDT, "the pipeline stages fit in the two tile buffers");
+static_assert(BT == FILL_TILE && BTH == FILL_THREADS && sizeof(FillTile) <= SMEM_DOUBLES * sizeof(double),
+              "a FILL task is one tile of the fill");
 constexpr size_t BATCH_SMEM = SMEM_DOUBLES * sizeof(double);
 
 enum BatchTaskType : int { TASK_FILL = 0, TASK_FACT = 1, TASK_FWD = 2, TASK_BWD = 3 };
@@ -143,45 +145,25 @@ __device__ __forceinline__ int* tile_flags(const BatchArgs& a, const tb_batch_it
 
 // ---------------------------------------------------------------- FILL
 __device__ void task_fill(const BatchArgs& a, const tb_batch_item_t& it, int i, int j, double* sm) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
   const int64_t N = it.N, T = it.T, Np = T * BT;
-  double* s_r = sm;
-  double* s_z = sm + BT * (NQ + 1);
-  double* s_w = sm + 2 * BT * (NQ + 1);
-  // the Gauss rings of the tile's 64 columns (the jacobian buffer's values)
-  for (int e = tid; e < BT * NQ; e += BTH) {
-    const int c = e / NQ, k = e % NQ;
-    const int64_t col = (int64_t)j * BT + c;
-    double r = 0, z = 0, w = 0;
-    if (col < N) {
-      Cubic cu;
-      cu.load(it.vertices + col * 12);
-      double jj;
-      cu.point(gauss_x(k), false, r, z, jj);
-      w = gauss_w(k) * jj;
-    }
-    s_r[c * (NQ + 1) + k] = r;
-    s_z[c * (NQ + 1) + k] = z;
-    s_w[c * (NQ + 1) + k] = w;
-  }
+  FillTile& s = *reinterpret_cast<FillTile*>(sm);
+  fill_columns(s, it.vertices, nullptr, nullptr, N, (int64_t)j * BT);
+  fill_rows(s, it.vertices, it.types, it.values, (int64_t)i * BT, N);
   __syncthreads();
   double* A = a.work + it.a_off;
+  const int c = tid % BT;
+  const int64_t col = (int64_t)j * BT + c;
 #pragma unroll 1
-  for (int aa = 0; aa < 4; aa++) {
-    const int64_t row = (int64_t)i * BT + ty + 16 * aa;
-#pragma unroll 1
-    for (int bb = 0; bb < 4; bb++) {
-      const int c = tx + 16 * bb;
-      const int64_t col = (int64_t)j * BT + c;
-      if (row == col && row < N) continue;  // self term below
-      double v;
-      if (row < N && col < N)
-        v = fill_entry(it.vertices, it.types, it.values, row, s_r + c * (NQ + 1), s_z + c * (NQ + 1),
-                       s_w + c * (NQ + 1));
-      else
-        v = row == col ? 1.0 : 0.0;
-      A[row * Np + col] = v;
-    }
+  for (int q = tid / BT; q < BT; q += BTH / BT) {
+    const int64_t row = (int64_t)i * BT + q;
+    if (row == col && row < N) continue;  // self term below
+    double v;
+    if (row < N && col < N)
+      v = fill_pair(s, q, c, it.vertices, nullptr, nullptr, col);
+    else
+      v = row == col ? 1.0 : 0.0;
+    A[row * Np + col] = v;
   }
   if (i == j) {
     const int warp = tid >> 5, lane = tid & 31;

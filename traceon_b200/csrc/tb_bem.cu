@@ -100,54 +100,53 @@ __global__ void k_element_targets(const double* __restrict__ vertices, double* _
 }
 
 // ---------------------------------------------------------------- fill
-// Block = 32 columns x 8 rows; the 32 columns' Gauss rings are staged in
-// shared memory once and reused by the 8 rows.
-constexpr int FILL_COLS = 32;
-constexpr int FILL_ROWS = 8;
+// One CTA per tile of 64 columns and up to 64 rows (fewer when the matrix is
+// small, launch_fill): the columns' quadrature nodes and the rows' collocation
+// data staged in shared memory (fill_columns, fill_rows), then thread (c, g)
+// walks rows g, g + 4, ... of column c: the 32 lanes of a warp write 256
+// contiguous bytes, and neighbouring columns mostly take the same rule.
+__device__ __forceinline__ void fill_tile(FillTile& s, double* __restrict__ A, int64_t lda,
+                                          const double* __restrict__ vertices, const uint8_t* __restrict__ types,
+                                          const double* __restrict__ values, const double* __restrict__ jac,
+                                          const double* __restrict__ pos, int64_t N, int64_t i0, int64_t i1, int64_t j0,
+                                          int accumulate, int gauss_diagonal) {
+  fill_columns(s, vertices, jac, pos, N, j0);
+  fill_rows(s, vertices, types, values, i0, i1);
+  __syncthreads();
+  const int c = threadIdx.x % FILL_TILE;
+  const int64_t j = j0 + c;
+  if (j < N) {
+#pragma unroll 1
+    for (int q = threadIdx.x / FILL_TILE; q < FILL_TILE && i0 + q < i1; q += FILL_THREADS / FILL_TILE) {
+      const int64_t i = i0 + q;
+      if (i == j && !gauss_diagonal) continue;
+      const double v = fill_pair(s, q, c, vertices, jac, pos, j);
+      double* a = A + i * lda + j;
+      *a = accumulate ? *a + v : v;
+    }
+  }
+}
 
-__global__ void __launch_bounds__(FILL_COLS* FILL_ROWS)
+__global__ void __launch_bounds__(FILL_THREADS)
     k_fill_matrix(double* __restrict__ A, int64_t lda, const double* __restrict__ vertices,
                   const uint8_t* __restrict__ types, const double* __restrict__ values,
                   const double* __restrict__ jac, const double* __restrict__ pos, int64_t N, int64_t row0,
-                  int64_t row1, int accumulate, int gauss_diagonal) {
-  __shared__ double s_r[FILL_COLS][NQ + 1], s_z[FILL_COLS][NQ + 1], s_w[FILL_COLS][NQ + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int64_t j0 = blockIdx.x * (int64_t)FILL_COLS;
-  const int tid = ty * FILL_COLS + tx;
-  for (int e = tid; e < FILL_COLS * NQ; e += FILL_COLS * FILL_ROWS) {
-    int c = e / NQ, k = e % NQ;
-    int64_t j = j0 + c;
-    double r = 0, z = 0, w = 0;
-    if (j < N) {
-      r = pos[(j * NQ + k) * 2];
-      z = pos[(j * NQ + k) * 2 + 1];
-      w = jac[j * NQ + k];
-    }
-    s_r[c][k] = r;
-    s_z[c][k] = z;
-    s_w[c][k] = w;
-  }
-  __syncthreads();
-  const int64_t i = row0 + blockIdx.y * (int64_t)FILL_ROWS + ty;
-  const int64_t j = j0 + tx;
-  if (i >= row1 || j >= N) return;
-  if (j == i && !gauss_diagonal) return;
-  const double acc = fill_entry(vertices, types, values, i, s_r[tx], s_z[tx], s_w[tx]);
-  double* a = A + (i * lda + j);
-  *a = accumulate ? *a + acc : acc;
+                  int64_t row1, int rows, int accumulate, int gauss_diagonal) {
+  __shared__ FillTile s;
+  const int64_t i0 = row0 + blockIdx.y * (int64_t)rows;
+  fill_tile(s, A, lda, vertices, types, values, jac, pos, N, i0, row1 - i0 < rows ? row1 : i0 + rows,
+            blockIdx.x * (int64_t)FILL_TILE, accumulate, gauss_diagonal);
 }
 
 // ---------------------------------------------------------------- batched fill
-// Many geometries of uneven N in one persistent launch: the tiles (32 columns
-// x 8 rows) of all matrices are numbered globally (geometry g owns tiles
-// [tile0[g], tile0[g] + tiles_x[g] tiles_y[g])); CTAs stride over them and
-// find their geometry by binary search.  Diagonal entries are left to the
-// self integrals, as in the single-geometry fill.
-__global__ void __launch_bounds__(FILL_COLS* FILL_ROWS)
+// Many geometries of uneven N in one persistent launch: the tiles of all
+// matrices are numbered globally (geometry g owns tiles [tile0[g], tile0[g] +
+// T^2), T = ceil(N / 64)); CTAs stride over them and find their geometry by
+// binary search.  Diagonal entries are left to the self integrals, as in the
+// single-geometry fill.
+__global__ void __launch_bounds__(FILL_THREADS)
     k_fill_matrix_batched(const tb_geometry_t* __restrict__ geoms, int n_geoms, int64_t total_tiles) {
-  __shared__ double s_r[FILL_COLS][NQ + 1], s_z[FILL_COLS][NQ + 1], s_w[FILL_COLS][NQ + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int tid = ty * FILL_COLS + tx;
+  __shared__ FillTile s;
   for (int64_t t = blockIdx.x; t < total_tiles; t += gridDim.x) {
     int lo = 0, hi = n_geoms - 1;  // last geometry with tile0 <= t
     while (lo < hi) {
@@ -158,27 +157,10 @@ __global__ void __launch_bounds__(FILL_COLS* FILL_ROWS)
         hi = mid - 1;
     }
     const tb_geometry_t& g = geoms[lo];
-    const int64_t N = g.N;
-    const int64_t tiles_x = (N + FILL_COLS - 1) / FILL_COLS;
-    const int64_t local = t - g.tile0;
-    const int64_t j0 = (local % tiles_x) * FILL_COLS, i0 = (local / tiles_x) * FILL_ROWS;
-    __syncthreads();  // the previous tile's rings are no longer read
-    for (int e = tid; e < FILL_COLS * NQ; e += FILL_COLS * FILL_ROWS) {
-      const int c = e / NQ, k = e % NQ;
-      const int64_t j = j0 + c;
-      double r = 0, z = 0, w = 0;
-      if (j < N) {
-        r = g.pos[(j * NQ + k) * 2];
-        z = g.pos[(j * NQ + k) * 2 + 1];
-        w = g.jac[j * NQ + k];
-      }
-      s_r[c][k] = r;
-      s_z[c][k] = z;
-      s_w[c][k] = w;
-    }
-    __syncthreads();
-    const int64_t i = i0 + ty, j = j0 + tx;
-    if (i < N && j < N && i != j) g.A[i * g.lda + j] = fill_entry(g.vertices, g.types, g.values, i, s_r[tx], s_z[tx], s_w[tx]);
+    const int64_t T = (g.N + FILL_TILE - 1) / FILL_TILE, local = t - g.tile0;
+    __syncthreads();  // the previous tile's data is no longer read
+    fill_tile(s, g.A, g.lda, g.vertices, g.types, g.values, g.jac, g.pos, g.N, (local / T) * FILL_TILE, g.N,
+              (local % T) * FILL_TILE, 0, 0);
   }
 }
 
@@ -601,10 +583,16 @@ extern "C" int tb_fill_matrix_radial(double* A, int64_t lda, const double* verti
   if (N < 0 || lda < N || row0 < 0 || row1 > N || row0 > row1) return BAD_ARG;
   if (N == 0 || row0 == row1) return OK;
   if (!A || !vertices || !types || !values || !jac || !pos) return BAD_ARG;
-  dim3 grid(unsigned((N + FILL_COLS - 1) / FILL_COLS), unsigned((row1 - row0 + FILL_ROWS - 1) / FILL_ROWS));
+  // Tall tiles share their columns' staging; a small matrix is cut lower until
+  // four CTAs per SM have work (101 elements: 15 us, 60 more with tiles of 64
+  // rows; from 3,072 elements on they are 64 rows high).
+  const int64_t gx = (N + FILL_TILE - 1) / FILL_TILE;
+  int rows = FILL_TILE;
+  while (rows > 4 && gx * ((row1 - row0 + rows - 1) / rows) < 4 * num_sms()) rows /= 2;
+  dim3 grid(unsigned(gx), unsigned((row1 - row0 + rows - 1) / rows));
   if (grid.y > 65535u) return BAD_ARG;
-  k_fill_matrix<<<grid, dim3(FILL_COLS, FILL_ROWS), 0, (cudaStream_t)stream>>>(
-      A, lda, vertices, types, values, jac, pos, N, row0, row1, accumulate, gauss_diagonal);
+  k_fill_matrix<<<grid, FILL_THREADS, 0, (cudaStream_t)stream>>>(
+      A, lda, vertices, types, values, jac, pos, N, row0, row1, rows, accumulate, gauss_diagonal);
   return launch_status();
 }
 
@@ -627,7 +615,7 @@ extern "C" int64_t tb_batch_plan(tb_geometry_t* geoms, int n_geoms, int64_t* tot
     if (N <= 0 || geoms[g].lda < N) return -1;
     geoms[g].tile0 = tiles;
     geoms[g].elem0 = elems;
-    tiles += ((N + FILL_COLS - 1) / FILL_COLS) * ((N + FILL_ROWS - 1) / FILL_ROWS);
+    tiles += ((N + FILL_TILE - 1) / FILL_TILE) * ((N + FILL_TILE - 1) / FILL_TILE);
     elems += N;
   }
   if (total_elements) *total_elements = elems;
@@ -640,8 +628,7 @@ extern "C" int tb_fill_matrix_radial_batched(const tb_geometry_t* geoms, int n_g
   // persistent: a few CTAs per SM stride over all tiles of all geometries
   int64_t blocks = (int64_t)num_sms() * 8;
   if (blocks > total_tiles) blocks = total_tiles;
-  k_fill_matrix_batched<<<unsigned(blocks), dim3(FILL_COLS, FILL_ROWS), 0, (cudaStream_t)stream>>>(geoms, n_geoms,
-                                                                                                  total_tiles);
+  k_fill_matrix_batched<<<unsigned(blocks), FILL_THREADS, 0, (cudaStream_t)stream>>>(geoms, n_geoms, total_tiles);
   return launch_status();
 }
 

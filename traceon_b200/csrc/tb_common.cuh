@@ -211,10 +211,10 @@ __device__ __forceinline__ double ring_pot_nopi(double r0, double z0, double rs,
   double rho2 = fma(dr, dr, dz2);
   double s = rs + r0;
   double D = fma(s, s, dz2);
-  double rD = rsqrt_nr(D);
+  double rD = rsqrt_h3(D);
   double t = rho2 * rD * rD;
   double t2 = t * t, t4 = t2 * t2;
-  double K = fma(-log_bf(t), estrin8(C_KB, t, t2, t4), estrin8(C_KA, t, t2, t4));
+  double K = fma(neglog_tab(t), estrin8(C_KB, t, t2, t4), estrin8(C_KA, t, t2, t4));
   return K * rs * rD;
 }
 
