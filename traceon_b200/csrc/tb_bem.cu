@@ -10,6 +10,8 @@
 //
 // Everything is FP64; the kernels are FP64-pipe bound (one log, one sqrt and
 // one division per ring pair).
+#include <cooperative_groups.h>
+
 #include "tb_common.cuh"
 #include "tb_internal.cuh"
 #include "tb_fill.cuh"
@@ -287,43 +289,81 @@ __global__ void __launch_bounds__(FP_THREADS)
   if (m < M) finish_field(p, Sr, Sz, Sp, pot, field, m);
 }
 
-// One team of TEAM threads (a warp or the whole block) per point.
-template <bool POT, int TEAM>
-__global__ void __launch_bounds__(TEAM >= 256 ? TEAM : 256)
-    k_field_points_team(const double* __restrict__ points, int64_t M, const double* __restrict__ src, int64_t Nq,
+// One warp per point.
+template <bool POT>
+__global__ void __launch_bounds__(256)
+    k_field_points_warp(const double* __restrict__ points, int64_t M, const double* __restrict__ src, int64_t Nq,
                         double* __restrict__ pot, double* __restrict__ field) {
-  constexpr int TEAMS = (TEAM >= 256 ? TEAM : 256) / TEAM;
-  int team = threadIdx.x / TEAM, lane = threadIdx.x % TEAM;
-  int64_t m = blockIdx.x * (int64_t)TEAMS + team;
-  double p[3] = {0, 0, 0};
-  if (m < M) {
-    p[0] = points[3 * m];
-    p[1] = points[3 * m + 1];
-    p[2] = points[3 * m + 2];
-  }
-  double r0 = axis_distance(p);
+  const int lane = threadIdx.x & 31;
+  const int64_t m = blockIdx.x * (int64_t)8 + threadIdx.x / 32;
+  if (m >= M) return;
+  const double p[3] = {points[3 * m], points[3 * m + 1], points[3 * m + 2]};
+  const double r0 = axis_distance(p);
   double Sr = 0, Sz = 0, Sp = 0;
-  if (m < M) source_sums<POT>(r0, p[2], src, Nq, lane, TEAM, Sr, Sz, Sp);
+  source_sums<POT>(r0, p[2], src, Nq, lane, 32, Sr, Sz, Sp);
   Sr = warp_sum(Sr);
   Sz = warp_sum(Sz);
   if (POT) Sp = warp_sum(Sp);
-  if (TEAM > 32) {
-    __shared__ double red[3][TEAM / 32 > 0 ? TEAM / 32 : 1];
-    int w = threadIdx.x / 32;
-    if ((threadIdx.x & 31) == 0) {
-      red[0][w] = Sr;
-      red[1][w] = Sz;
-      red[2][w] = Sp;
-    }
-    __syncthreads();
-    Sr = Sz = Sp = 0;
-    for (int k = 0; k < TEAM / 32; k++) {
-      Sr += red[0][k];
-      Sz += red[1][k];
-      Sp += red[2][k];
-    }
+  if (lane == 0) finish_field(p, Sr, Sz, Sp, pot, field, m);
+}
+
+// One cluster of CTAs (1, 2, 4 or 8) per point, for a few points: a CTA alone
+// would leave the other SMs idle for as long as its 256 threads take (one
+// point on 16,000 rings: 35 us with one CTA, 6 with eight).  Each CTA's sums
+// go to the first one's shared memory and are added there in a fixed order.
+constexpr int FP_CLUSTER = 8;
+template <bool POT>
+__global__ void __launch_bounds__(256)
+    k_field_points_cluster(const double* __restrict__ points, const double* __restrict__ src, int64_t Nq,
+                           double* __restrict__ pot, double* __restrict__ field) {
+  namespace cg = cooperative_groups;
+  __shared__ double red[8][3], all[FP_CLUSTER][3];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ctas = int(cl.num_blocks()), rank = int(cl.block_rank());
+  const int64_t m = blockIdx.x / ctas;
+  const double p[3] = {points[3 * m], points[3 * m + 1], points[3 * m + 2]};
+  const double r0 = axis_distance(p);
+  double S[3] = {0, 0, 0};
+  source_sums<POT>(r0, p[2], src, Nq, rank * 256 + threadIdx.x, 256 * ctas, S[0], S[1], S[2]);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const double v = k < 2 || POT ? warp_sum(S[k]) : 0.0;
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x / 32][k] = v;
   }
-  if (m < M && lane == 0) finish_field(p, Sr, Sz, Sp, pot, field, m);
+  __syncthreads();
+  cl.sync();  // every CTA of the cluster runs: its shared memory can be written
+  if (threadIdx.x < 3) {
+    double t = 0;
+    for (int k = 0; k < 8; k++) t += red[k][threadIdx.x];
+    *cl.map_shared_rank(&all[rank][threadIdx.x], 0) = t;
+  }
+  cl.sync();
+  if (rank == 0 && threadIdx.x == 0) {
+    double t[3] = {0, 0, 0};
+    for (int c = 0; c < ctas; c++)
+      for (int k = 0; k < 3; k++) t[k] += all[c][k];
+    finish_field(p, t[0], t[1], t[2], pot, field, m);
+  }
+}
+
+template <bool POT>
+static void launch_points_cluster(const double* points, int64_t M, const double* src, int64_t Nq, double* pot,
+                                  double* field, cudaStream_t s) {
+  // as many CTAs a point as leave every point's cluster a place on the chip at
+  // once and every thread four rings
+  unsigned ctas = 1;
+  while (ctas < FP_CLUSTER && M * ctas * 2 <= num_sms() && Nq >= int64_t(ctas) * 2 * 256 * 4) ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(M) * ctas);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_field_points_cluster<POT>, points, src, Nq, pot, field);  // errors: launch_status()
 }
 
 // ---------------------------------------------------------------- axial
@@ -386,9 +426,9 @@ __global__ void k_axial_quintic(const double* __restrict__ d, int64_t Nz, double
 }
 
 // Not-a-knot cubic spline (scipy.interpolate.CubicSpline default) of the
-// columns 7 and 8 of d, one block per column.  Unknowns are the node slopes
-// s_0 .. s_{n-1}; on an equal grid with m_i = (y_{i+1} - y_i)/h:
-//   s_{i-1} + 4 s_i + s_{i+1} = 3 (m_{i-1} + m_i),      0 < i < n-1
+// columns 7 and 8 of d.  Unknowns are the node slopes s_0 .. s_{n-1}; on an
+// equal grid with m_i = (y_{i+1} - y_i)/h:
+//   s_{i-1} + 4 s_i + s_{i+1} = r_i = 3 (m_{i-1} + m_i),      0 < i < n-1
 //   not-a-knot at x_1:      s_0 - s_2 = 2 (m_0 - m_1)
 //   not-a-knot at x_{n-2}:  s_{n-1} - s_{n-3} = 2 (m_{n-2} - m_{n-3})
 // Eliminating s_0 and s_{n-1} leaves a tridiagonal system in s_1..s_{n-2}
@@ -737,7 +777,7 @@ extern "C" int tb_field_radial_points(const double* points, int64_t M, const dou
   cudaStream_t s = (cudaStream_t)stream;
   const int sms = num_sms();
   // Enough points to fill the GPU one thread per point: stage sources in
-  // shared memory.  Otherwise split each point's sum over a warp or a block.
+  // shared memory.  Otherwise split each point's sum over a warp or a cluster.
   if (M >= (int64_t)sms * 2048) {
     unsigned g = unsigned((M + FP_THREADS - 1) / FP_THREADS);
     if (pot)
@@ -747,15 +787,13 @@ extern "C" int tb_field_radial_points(const double* points, int64_t M, const dou
   } else if (M >= (int64_t)sms * 16) {
     unsigned g = unsigned((M + 7) / 8);
     if (pot)
-      k_field_points_team<true, 32><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
+      k_field_points_warp<true><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
     else
-      k_field_points_team<false, 32><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
+      k_field_points_warp<false><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
+  } else if (pot) {
+    launch_points_cluster<true>(points, M, sources, Nq, pot, field, s);
   } else {
-    unsigned g = unsigned(M);
-    if (pot)
-      k_field_points_team<true, 256><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
-    else
-      k_field_points_team<false, 256><<<g, 256, 0, s>>>(points, M, sources, Nq, pot, field);
+    launch_points_cluster<false>(points, M, sources, Nq, pot, field, s);
   }
   return launch_status();
 }
