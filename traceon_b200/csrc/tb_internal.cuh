@@ -69,6 +69,11 @@ inline int num_sms() {
 // spaced grid zi and evaluate the derivative polynomials first .. 8 (the
 // field needs 1 .. 8, the potential 0, 2, 4, 6, 8).  Returns false outside
 // [zi[0], zi[Nz-1]].
+//
+// On the device every thread reads its own interval's rows, so a warp's loads
+// touch 32 lines each and are bound by the L1's tag lookups, not by bytes:
+// a row's six coefficients are read as three pairs (rows start at multiples
+// of 48 bytes; a table that is not 16-byte aligned takes single loads).
 __host__ __device__ inline bool axial_eval(double z, const double* zi, const double* coeff, int64_t Nz,
                                            double* d, int first = 0) {
   double z0 = zi[0], zl = zi[Nz - 1];
@@ -79,7 +84,21 @@ __host__ __device__ inline bool axial_eval(double z, const double* zi, const dou
   if (idx > Nz - 2) idx = Nz - 2;
   double x = z - zi[idx];
   const double* C = coeff + idx * NDERIV * 6;
-  for (int i = first; i < NDERIV; i++) {
+#ifdef __CUDA_ARCH__
+  if ((reinterpret_cast<uintptr_t>(coeff) & 15) == 0) {
+#pragma unroll
+    for (int i = 0; i < NDERIV; i++) {
+      if (i < first) continue;
+      const double2* c = reinterpret_cast<const double2*>(C + i * 6);
+      const double2 a = c[0], b = c[1], e = c[2];
+      d[i] = ((((a.x * x + a.y) * x + b.x) * x + b.y) * x + e.x) * x + e.y;
+    }
+    return true;
+  }
+#pragma unroll
+#endif
+  for (int i = 0; i < NDERIV; i++) {
+    if (i < first) continue;
     const double* c = C + i * 6;
     d[i] = ((((c[0] * x + c[1]) * x + c[2]) * x + c[3]) * x + c[4]) * x + c[5];
   }
