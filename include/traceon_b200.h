@@ -565,6 +565,17 @@ int tb_mlp_colsum(const void *dZ, float *db, int64_t M, int64_t N, tb_stream_t s
  * BF16 copy pb. */
 int tb_mlp_adam(float *p, const float *g, float *m, float *v, void *pb, int64_t n, float lr, float b1, float b2,
                 float eps, int64_t step, tb_stream_t stream);
+/* Loss and gradients of a batch in one pass: X (M x 16) BF16 features, T (M x
+ * n_out) targets, w (M) sample weights or NULL, weights_bf16 (16-byte aligned)
+ * and params_f32 the flat parameters (the biases are read from the FP32 copy).
+ * grad (all parameters, FP32) and *loss (device) = the mean over M n_out of
+ * w (Y - T)^2.  The same roundings as the single kernels above; the sums over
+ * the batch in a fixed order.  work: tb_mlp_loss_grad_workspace(M) bytes,
+ * 16-byte aligned. */
+int64_t tb_mlp_loss_grad_workspace(int64_t M);
+int tb_mlp_loss_grad(const void *X, const float *T, const float *w, int64_t M, int64_t n_out, const void *weights_bf16,
+                     const float *params_f32, float *grad, float *loss, void *work, int64_t work_bytes,
+                     tb_stream_t stream);
 /* Input features (M x 16, BF16) of M points (M,3): rho = r / r_max,
  * zeta = (z - z_c) / z_half. */
 int tb_mlp_features(const double *points, int64_t M, double r_max, double z_c, double z_half, void *X,

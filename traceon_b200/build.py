@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, 'libtraceon_b200.so')
 INCLUDE = os.path.join(os.path.dirname(HERE), 'include')
 
 SOURCES = ['tb_bem.cu', 'tb_lu.cu', 'tb_trace.cu', 'tb_compat.cu', 'tb_mlp.cu', 'tb_lu_mixed.cu', 'tb_post.cu', 'tb_batch.cu',
-           'tb_tree.cu']
+           'tb_tree.cu', 'tb_mlp_train.cu']
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 FLAGS = ['-O3', '-lineinfo', '-std=c++17', '-Xcompiler', '-fPIC', '-shared', '--expt-relaxed-constexpr',
          '-Xptxas', '-v']

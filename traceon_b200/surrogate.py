@@ -51,10 +51,13 @@ for _name, _args in {
     'tb_mlp_silu_back': (_vp, _vp, _vp, _i64, _vp),
     'tb_mlp_colsum': (_vp, _vp, _i64, _i64, _vp),
     'tb_mlp_adam': (_vp, _vp, _vp, _vp, _vp, _i64, _f, _f, _f, _f, _i64, _vp),
+    'tb_mlp_loss_grad': (_vp, _vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp, _vp, _i64, _vp),
     'tb_mlp_features': (_vp, _i64, C.c_double, C.c_double, C.c_double, _vp, _vp),
 }.items():
     getattr(_lib, _name).argtypes = list(_args)
     getattr(_lib, _name).restype = C.c_int
+_lib.tb_mlp_loss_grad_workspace.argtypes = [_i64]
+_lib.tb_mlp_loss_grad_workspace.restype = _i64
 
 
 class TbSurrogate(C.Structure):
@@ -128,33 +131,16 @@ class MLP:
 
     def loss_and_grad(self, X, T, n_out, w=None):
         """MSE over the first n_out outputs (rows weighted by w (M) if given);
-        fills self.g, returns the loss (device scalar)."""
+        fills self.g, returns the loss (device scalar).  One kernel for the
+        whole pass and one for the sums over its blocks (tb_mlp_loss_grad)."""
         torch = B._torch()
         M = X.shape[0]
-        out, pre, acts = self.forward(X, keep=True)
-        dY = torch.empty((M, OUT), dtype=torch.bfloat16, device=X.device)
-        nblk = (M * OUT + 255) // 256
-        part = torch.empty(nblk, dtype=torch.float32, device=X.device)
-        _call('tb_mlp_mse_grad', out.data_ptr(), T.data_ptr(), B._ptr(w), dY.data_ptr(), part.data_ptr(), M, OUT,
-              n_out, _s())
-        g = dY
-        for li in range(len(LAYERS) - 1, -1, -1):
-            W, b, fin, fout = LAYERS[li]
-            Xin = acts[li]
-            # dW = g^T . Xin  (fout x fin), db = column sums of g
-            _call('tb_mlp_gemm', g.data_ptr(), fout, 1, Xin.data_ptr(), fin, 1, self._w(self.g, W).data_ptr(), fin,
-                  fout, fin, M, 0, _s())
-            _call('tb_mlp_colsum', g.data_ptr(), self._w(self.g, b).data_ptr(), M, fout, _s())
-            if li == 0:
-                break
-            # dA = g . W  (M x fin), then through SiLU of layer li-1
-            dA = torch.empty((M, fin), dtype=torch.float32, device=X.device)
-            _call('tb_mlp_gemm', g.data_ptr(), fout, 0, self._w(self.pb, W).data_ptr(), fin, 1, dA.data_ptr(), fin,
-                  M, fin, fout, 0, _s())
-            gz = torch.empty((M, fin), dtype=torch.bfloat16, device=X.device)
-            _call('tb_mlp_silu_back', dA.data_ptr(), pre[li - 1].data_ptr(), gz.data_ptr(), M * fin, _s())
-            g = gz
-        return part.sum() / (M * n_out)
+        loss = torch.empty((), dtype=torch.float32, device=X.device)
+        nbytes = _lib.tb_mlp_loss_grad_workspace(M)
+        work = torch.empty(nbytes, dtype=torch.uint8, device=X.device)
+        _call('tb_mlp_loss_grad', X.data_ptr(), T.data_ptr(), B._ptr(w), M, n_out, self.pb.data_ptr(),
+              self.p.data_ptr(), self.g.data_ptr(), loss.data_ptr(), work.data_ptr(), nbytes, _s())
+        return loss
 
     def adam(self, lr, b1=0.9, b2=0.999, eps=1e-8):
         self.step_count += 1
