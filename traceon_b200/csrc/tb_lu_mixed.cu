@@ -175,74 +175,61 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------- FP32 panel kernels
-// Panel kernels of lu_nopiv_f32_tc (64-wide blocks).
+// The panel kernels of lu_nopiv_f32_tc.  The factorisation's critical path is
+// its chain of 64-column steps (256 of them at N = 16,384), each of which was
+// four dependent launches: the diagonal block's LU on one CTA (17 us), the
+// triangular solves below and right of it (15 + 10 us), and the panel's update
+// (16 to 29 us).  k_panel_step does all four in one launch: every CTA factors
+// the 64 x 64 diagonal block for itself (reading 16 KB beats waiting for
+// another launch), solves the panel's row block and its own 128 rows, and
+// updates its rows of the panel, in FP32.  That pays as long as all CTAs of a
+// step run at once (each repeats the block's LU); taller panels, of which the
+// SMs left free of the trailing update hold only a part, keep the separate
+// kernels, with the update on the tensor cores (118 us a step at N = 16,384
+// with k_panel_step for all panels, some 80 so).  k_row_block then solves the
+// rest of the panel's 256 rows in one launch instead of eight.  Solve of 2,501
+// elements 7.4 -> 4.4 ms, of 301 elements 777 -> 475 us of device time (with
+// k_diag_inverse, below), of 16,384 elements 60 -> 56 ms.
+//
+// CTAs of a step must not see the row block and the diagonal block change
+// under them, so CTA 0 puts these two into a scratch area (PanelScratch);
+// k_row_block, or k_panel_store after the last panel, moves them into A.
+constexpr int PS_ROWS = 128;      // rows of a CTA
+constexpr int PS_THREADS = 320;   // 4 warps on the rows' solves, 6 on the row block's
+constexpr int PS_COLS = 192;      // columns of the panel right of a step's block
+constexpr int PS_VLD = PS_ROWS + 1;
+constexpr int PS_CLD = MX_NB + 4;
+constexpr int TC_PANEL = 256;
 
-// D (the nb x nb diagonal block at (k0, k0)) <- its LU factors in place.
-// Thread t owns column j = t % 64 of rows t / 64 + 4 s (s = 0..15) in
-// registers; at step k the owners publish column k and row k to shared
-// memory (double-buffered by the parity of k: one barrier per step) and
-// every thread updates its elements with the pivot's reciprocal.  Fully
-// unrolled (k and s are constants in every iteration, so no dynamic
-// register indexing).  Rows and columns beyond nb are the identity.
-__global__ void __launch_bounds__(256) k_diag_lu_f32(float* __restrict__ A, int64_t lda, int64_t k0, int nb) {
-  pdl_wait();
-  __shared__ float colk[2][MX_NB], rowk[2][MX_NB];
-  const int j = threadIdx.x % MX_NB, i0 = threadIdx.x / MX_NB;
-  float v[16];
-#pragma unroll
-  for (int sI = 0; sI < 16; sI++) {
-    const int i = i0 + 4 * sI;
-    v[sI] = (i < nb && j < nb) ? A[(k0 + i) * lda + k0 + j] : (i == j ? 1.f : 0.f);
-  }
-#pragma unroll
-  for (int k = 0; k < MX_NB - 1; k++) {
-    if (k >= nb - 1) break;
-    const int buf = k & 1;
-    if (j == k) {
-#pragma unroll
-      for (int sI = 0; sI < 16; sI++) colk[buf][i0 + 4 * sI] = v[sI];
-    }
-    if (i0 == (k & 3)) rowk[buf][j] = v[k >> 2];
-    __syncthreads();
-    const float inv = 1.f / rowk[buf][k];
-    const float u = rowk[buf][j];
-#pragma unroll
-    for (int sI = 0; sI < 16; sI++) {
-      const int i = i0 + 4 * sI;
-      if (i > k) {
-        const float l = colk[buf][i] * inv;
-        if (j == k)
-          v[sI] = l;
-        else if (j > k)
-          v[sI] = fmaf(-l, u, v[sI]);
-      }
-    }
-  }
-#pragma unroll
-  for (int sI = 0; sI < 16; sI++) {
-    const int i = i0 + 4 * sI;
-    if (i < nb && j < nb) A[(k0 + i) * lda + k0 + j] = v[sI];
-  }
-}
+struct PanelScratch {  // one 64-column step
+  float d[MX_NB][MX_NB];     // the factored diagonal block
+  float u[MX_NB][PS_COLS];   // the panel's row block right of it
+};
+
+struct PanelSmem {
+  float U[MX_NB][PS_CLD];    // upper factor, reciprocal pivots on its diagonal
+  float Lt[MX_NB][PS_CLD];   // lower factor, transposed
+  float V[MX_NB][PS_VLD];    // V[m][r]: element m of row r of the CTA
+  float W[MX_NB][PS_COLS];   // W[i][c]: row i of column c of the row block
+  float colk[2][MX_NB], rowk[2][MX_NB];
+};
 
 // Forward substitution on the 64-long vectors V[.][t] (one per thread, in
-// shared memory, V[m][t] = element m): x_i = (v_i - sum_{p < i} C[p][i] x_p)
-// times C[i][i] when DIAG (the caller stores the reciprocal pivots on the
-// diagonal of C), unit diagonal otherwise.  Blocked by 8: the 8 unknowns of
-// a block stay in registers while every finished unknown p < block is
-// applied to all 8 (two 16-byte broadcast reads of C per p), then the block
-// is solved in registers.
-constexpr int TRSM_COLS = 128;
+// shared memory, V[m * ld + t] = element m): x_i = (v_i - sum_{p < i} C[p][i]
+// x_p) times C[i][i] when DIAG (reciprocal pivots on the diagonal of C), unit
+// diagonal otherwise.  Blocked by 8: the 8 unknowns of a block stay in
+// registers while every finished unknown p < block is applied to all 8 (two
+// 16-byte broadcast reads of C per p), then the block is solved in registers.
 template <bool DIAG>
-__device__ __forceinline__ void solve_vectors(float (*V)[TRSM_COLS], const float (*C)[MX_NB], int t) {
+__device__ __forceinline__ void solve_vectors(float* V, int ld, const float (*C)[PS_CLD]) {
 #pragma unroll 1
   for (int b0 = 0; b0 < MX_NB; b0 += 8) {
     float x[8];
 #pragma unroll
-    for (int c = 0; c < 8; c++) x[c] = V[b0 + c][t];
+    for (int c = 0; c < 8; c++) x[c] = V[(b0 + c) * ld];
 #pragma unroll 4
     for (int p = 0; p < b0; p++) {
-      const float xp = V[p][t];
+      const float xp = V[p * ld];
       const float4 c0 = *reinterpret_cast<const float4*>(&C[p][b0]);
       const float4 c1 = *reinterpret_cast<const float4*>(&C[p][b0 + 4]);
       x[0] = fmaf(-c0.x, xp, x[0]);
@@ -259,10 +246,190 @@ __device__ __forceinline__ void solve_vectors(float (*V)[TRSM_COLS], const float
 #pragma unroll
       for (int q = 0; q < c; q++) x[c] = fmaf(-C[b0 + q][b0 + c], x[q], x[c]);
       if (DIAG) x[c] *= C[b0 + c][b0 + c];
-      V[b0 + c][t] = x[c];
+      V[(b0 + c) * ld] = x[c];
     }
   }
 }
+
+// LU of the 64 x 64 block whose rows t / 64 + 4 q (q = 0..15) of column t % 64
+// are v[q] of thread t < 256 (named barrier 1): at step k the owners publish
+// column k (zeros down to row k; thread group g's rows at 16 g) and row k
+// (double-buffered by the parity of k: one barrier per step) and every thread
+// takes column k times its element of row k over the pivot off its own.  The
+// four steps that share a register index q run the same code: unrolled over
+// all 64 steps the kernel is bound by fetching instructions that it runs once
+// (16 us a block; 18 us unrolled over 16 steps, 40 us over 64).
+__device__ __forceinline__ void block_lu(float (&v)[16], float (*colk)[MX_NB], float (*rowk)[MX_NB]) {
+  const int j = threadIdx.x % MX_NB, g = threadIdx.x / MX_NB;
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+#pragma unroll 1
+    for (int gg = 0; gg < (q < 15 ? 4 : 3); gg++) {
+      const int k = 4 * q + gg, buf = gg & 1;
+      if (j == k) {
+#pragma unroll
+        for (int w = q / 4; w < 4; w++) {
+          float f[4];
+#pragma unroll
+          for (int z = 0; z < 4; z++) {
+            const int r = 4 * w + z;
+            f[z] = r > q ? v[r] : (r == q && g > gg ? v[r] : 0.f);
+          }
+          *reinterpret_cast<float4*>(&colk[buf][16 * g + 4 * w]) = make_float4(f[0], f[1], f[2], f[3]);
+        }
+      }
+      if (g == gg) rowk[buf][j] = v[q];
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      const float p = rowk[buf][k], rj = rowk[buf][j];
+      float c[16];
+#pragma unroll
+      for (int w = q / 4; w < 4; w++) {
+        const float4 f = *reinterpret_cast<const float4*>(&colk[buf][16 * g + 4 * w]);
+        c[4 * w] = f.x;
+        c[4 * w + 1] = f.y;
+        c[4 * w + 2] = f.z;
+        c[4 * w + 3] = f.w;
+      }
+      float inv;  // 1 / p: the hardware approximation and one Newton step
+      asm("rcp.approx.f32 %0, %1;" : "=f"(inv) : "f"(p));
+      inv = fmaf(inv, fmaf(-p, inv, 1.f), inv);
+      const bool here = j == k;
+      const float u = here ? inv : (j > k ? -rj * inv : 0.f);  // column k itself becomes the multipliers
+      if (g > gg) v[q] = fmaf(c[q], u, here ? 0.f : v[q]);
+#pragma unroll
+      for (int r = q + 1; r < 16; r++) v[r] = fmaf(c[r], u, here ? 0.f : v[r]);
+    }
+  }
+}
+
+// The nb x nb block at (k0, k0) (rows and columns beyond nb: the identity)
+// factored into s.U and s.Lt by 256 threads, and into keep unless null.
+__device__ __forceinline__ void panel_diag_lu(PanelSmem& s, const float* __restrict__ A, int64_t lda, int64_t k0, int nb,
+                                              float* __restrict__ keep) {
+  const int t = threadIdx.x, j = t % MX_NB, g = t / MX_NB;
+  float v[16];
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int i = g + 4 * q;
+    v[q] = (i < nb && j < nb) ? A[(k0 + i) * lda + k0 + j] : (i == j ? 1.f : 0.f);
+  }
+  block_lu(v, s.colk, s.rowk);
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int i = g + 4 * q;
+    if (i <= j) s.U[i][j] = i == j ? __frcp_rn(v[q]) : v[q];
+    s.Lt[j][i] = i > j ? v[q] : 0.f;
+    if (keep) keep[i * MX_NB + j] = v[q];
+  }
+}
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(in ? 4 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_all() {
+  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+}
+
+// The solves and the CTA's rows of the update, C -= V^T W over 16 NJ columns:
+// 256 threads, 8 x NJ outputs each, read before the solves.
+template <int NJ>
+__device__ __forceinline__ void panel_solve_update(PanelSmem& s, float* __restrict__ C, int64_t lda, int rows, int right) {
+  const int t = threadIdx.x, tr = t / 16, tc = t % 16;
+  float acc[8][NJ > 0 ? NJ : 1];
+  if (NJ > 0 && t < 256) {
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j < NJ; j++)
+        acc[i][j] = (tr + 16 * i < rows && tc + 16 * j < right) ? C[(tr + 16 * i) * lda + tc + 16 * j] : 0.f;
+  }
+  if (t < PS_ROWS)
+    solve_vectors<true>(&s.V[0][t], PS_VLD, s.U);
+  else if (t - PS_ROWS < right)
+    solve_vectors<false>(&s.W[0][t - PS_ROWS], PS_COLS, s.Lt);
+  __syncthreads();
+  if (NJ > 0 && t < 256) {
+#pragma unroll 2
+    for (int m = 0; m < MX_NB; m++) {
+      float a[8], b[NJ > 0 ? NJ : 1];
+#pragma unroll
+      for (int i = 0; i < 8; i++) a[i] = s.V[m][tr + 16 * i];
+#pragma unroll
+      for (int j = 0; j < NJ; j++) b[j] = s.W[m][tc + 16 * j];
+#pragma unroll
+      for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j < NJ; j++) acc[i][j] = fmaf(-a[i], b[j], acc[i][j]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j < NJ; j++)
+        if (tr + 16 * i < rows && tc + 16 * j < right) C[(tr + 16 * i) * lda + tc + 16 * j] = acc[i][j];
+  }
+}
+
+// Columns k0 .. k0 + nb - 1 of the panel that ends at column pe.
+__global__ void __launch_bounds__(PS_THREADS, 1)
+    k_panel_step(float* __restrict__ A, int64_t lda, int64_t N, int64_t k0, int nb, int64_t pe,
+                 PanelScratch* __restrict__ scratch) {
+  extern __shared__ __align__(16) unsigned char ps_raw[];
+  PanelSmem& s = *reinterpret_cast<PanelSmem*>(ps_raw);
+  pdl_wait();
+  const int tid = threadIdx.x;
+  const int64_t r0 = k0 + nb + blockIdx.x * (int64_t)PS_ROWS;
+  const int rows = r0 >= N ? 0 : (N - r0 < PS_ROWS ? int(N - r0) : PS_ROWS);
+  const int right = int(pe - k0 - nb);
+  // this CTA's rows (transposed) and the row block, arriving during the LU
+  for (int e = tid; e < PS_ROWS * MX_NB; e += PS_THREADS) {
+    const int r = e / MX_NB, m = e % MX_NB;
+    const bool in = r < rows && m < nb;
+    cp_async4(&s.V[m][r], in ? A + (r0 + r) * lda + k0 + m : A, in);
+  }
+  for (int c = tid % 32; c < right; c += 32)
+    for (int i = tid / 32; i < MX_NB; i += PS_THREADS / 32)
+      cp_async4(&s.W[i][c], i < nb ? A + (k0 + i) * lda + k0 + nb + c : A, i < nb);
+  if (tid < 256) panel_diag_lu(s, A, lda, k0, nb, blockIdx.x == 0 ? &scratch->d[0][0] : nullptr);
+  cp_async_all();
+  __syncthreads();
+  float* C = A + r0 * lda + k0 + nb;
+  if (right > 128)
+    panel_solve_update<12>(s, C, lda, rows, right);
+  else if (right > 64)
+    panel_solve_update<8>(s, C, lda, rows, right);
+  else if (right > 0)
+    panel_solve_update<4>(s, C, lda, rows, right);
+  else
+    panel_solve_update<0>(s, C, lda, rows, right);
+  if (blockIdx.x == 0)
+    for (int e = tid; e < MX_NB * PS_COLS; e += PS_THREADS)
+      if (e % PS_COLS < right) (&scratch->u[0][0])[e] = (&s.W[0][0])[e];
+  for (int e = tid; e < rows * MX_NB; e += PS_THREADS) {
+    const int r = e / MX_NB, m = e % MX_NB;
+    if (m < nb) A[(r0 + r) * lda + k0 + m] = s.V[m][r];
+  }
+}
+
+// The separate kernels of a tall panel's step.
+__global__ void __launch_bounds__(256) k_diag_lu_f32(float* __restrict__ A, int64_t lda, int64_t k0, int nb) {
+  pdl_wait();
+  __shared__ __align__(16) float colk[2][MX_NB], rowk[2][MX_NB];
+  const int t = threadIdx.x, j = t % MX_NB, g = t / MX_NB;
+  float v[16];
+#pragma unroll
+  for (int q = 0; q < 16; q++) {
+    const int i = g + 4 * q;
+    v[q] = (i < nb && j < nb) ? A[(k0 + i) * lda + k0 + j] : (i == j ? 1.f : 0.f);
+  }
+  block_lu(v, colk, rowk);
+#pragma unroll
+  for (int q = 0; q < 16; q++)
+    if (g + 4 * q < nb && j < nb) A[(k0 + g + 4 * q) * lda + k0 + j] = v[q];
+}
+
+constexpr int TRSM_COLS = 128;
+constexpr int TRSM_SMEM = MX_NB * TRSM_COLS * int(sizeof(float));
 
 // rows r0 <= i < r1: A[i, k0:k0+nb] <- A[i, k0:k0+nb] U11^-1.  x U = a is
 // x_m = (a_m - sum_{p < m} x_p U[p][m]) / U[m][m]: solve_vectors with
@@ -272,8 +439,9 @@ __device__ __forceinline__ void solve_vectors(float (*V)[TRSM_COLS], const float
 __global__ void __launch_bounds__(TRSM_COLS)
     k_trsm_right_f32(float* __restrict__ A, int64_t lda, int64_t r0, int64_t r1, int64_t k0, int nb) {
   pdl_wait();
-  __shared__ __align__(16) float U[MX_NB][MX_NB];
-  __shared__ float V[MX_NB][TRSM_COLS];  // V[m][r]: element m of row r of the CTA
+  __shared__ __align__(16) float U[MX_NB][PS_CLD];
+  extern __shared__ __align__(16) float tr_V[];
+  float(*V)[TRSM_COLS] = reinterpret_cast<float(*)[TRSM_COLS]>(tr_V);  // V[m][r]: element m of row r of the CTA
   const int64_t rb = r0 + blockIdx.x * (int64_t)TRSM_COLS;
   const int nrow = r1 - rb < TRSM_COLS ? int(r1 - rb) : TRSM_COLS;
   const int r = threadIdx.x;  // lanes over rows: conflict-free shared stores
@@ -309,7 +477,7 @@ __global__ void __launch_bounds__(TRSM_COLS)
     }
   }
   __syncthreads();
-  solve_vectors<true>(V, U, r);
+  solve_vectors<true>(&V[0][r], TRSM_COLS, U);
   if (r < nrow) {
     if (vec) {
 #pragma unroll
@@ -329,8 +497,9 @@ __global__ void __launch_bounds__(TRSM_COLS)
 __global__ void __launch_bounds__(TRSM_COLS)
     k_trsm_left_f32(float* __restrict__ A, int64_t lda, int64_t c0, int64_t c1, int64_t k0, int nb) {
   pdl_wait();
-  __shared__ __align__(16) float Lt[MX_NB][MX_NB];
-  __shared__ float V[MX_NB][TRSM_COLS];  // V[i][c]: row i of column c of the CTA
+  __shared__ __align__(16) float Lt[MX_NB][PS_CLD];
+  extern __shared__ __align__(16) float tr_V[];
+  float(*V)[TRSM_COLS] = reinterpret_cast<float(*)[TRSM_COLS]>(tr_V);  // V[i][c]: row i of column c of the CTA
   const int64_t cb = c0 + blockIdx.x * (int64_t)TRSM_COLS;
   const int ncol = c1 - cb < TRSM_COLS ? int(c1 - cb) : TRSM_COLS;
   {
@@ -352,9 +521,172 @@ __global__ void __launch_bounds__(TRSM_COLS)
     }
   }
   __syncthreads();
-  solve_vectors<false>(V, Lt, threadIdx.x);
+  solve_vectors<false>(&V[0][threadIdx.x], TRSM_COLS, Lt);
   for (int ii = 0; ii < nb; ii++)
     if (threadIdx.x < ncol) A[(k0 + ii) * lda + cb + threadIdx.x] = V[ii][threadIdx.x];
+}
+
+// Moves a panel's diagonal and row blocks from the scratch area into A (all
+// CTAs of the grid take part).
+__device__ __forceinline__ void panel_store(float* __restrict__ A, int64_t lda, int64_t p0, int64_t pe,
+                                            const PanelScratch* __restrict__ scratch) {
+  const int first = int(blockIdx.x * blockDim.x + threadIdx.x), step = int(gridDim.x * blockDim.x);
+  for (int64_t k0 = p0; k0 < pe; k0 += MX_NB, scratch++) {
+    const int nb = pe - k0 < MX_NB ? int(pe - k0) : MX_NB, width = int(pe - k0);
+    for (int e = first; e < nb * width; e += step) {
+      const int i = e / width, j = e % width;
+      A[(k0 + i) * lda + k0 + j] = j < nb ? scratch->d[i][j] : scratch->u[i][j - nb];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256) k_panel_store(float* __restrict__ A, int64_t lda, int64_t p0, int64_t pe,
+                                                     const PanelScratch* __restrict__ scratch) {
+  pdl_wait();
+  panel_store(A, lda, p0, pe, scratch);
+}
+
+// The row block right of a full panel: U12 = L11^-1 A12 for rows p0 .. p0 +
+// 255, 64 columns a CTA, all in shared memory: for each 64 rows the
+// triangular solve (16 rows at a time: one thread per column within them, all
+// threads for the rest of the 64), then their product with the panel's rows
+// below taken off the rest.  The panel's blocks arrive one step ahead.
+constexpr int RB_COLS = 64;
+constexpr int RB_THREADS = 256;
+constexpr int RB_LLD = 192 + 4;
+struct RowBlockSmem {
+  float X[TC_PANEL][RB_COLS];
+  float L[2][MX_NB][RB_LLD];     // L[m][r]: element m of row r of the rows below
+  float Lt[2][MX_NB][PS_CLD];    // the diagonal block's L transposed: Lt[m][i] = L[i][m]
+};
+
+// X_b <- L_bb^-1 X_b for the 64 rows at Xb.
+__device__ __forceinline__ void row_block_solve(float (*Xb)[RB_COLS], const float (*Lt)[PS_CLD]) {
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+#pragma unroll 1
+  for (int s0 = 0; s0 < MX_NB; s0 += 16) {
+    if (threadIdx.x < RB_COLS) {
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; i++) x[i] = Xb[s0 + i][threadIdx.x];
+#pragma unroll
+      for (int m = 0; m < 15; m++)
+#pragma unroll
+        for (int i = m + 1; i < 16; i++) x[i] = fmaf(-Lt[s0 + m][s0 + i], x[m], x[i]);
+#pragma unroll
+      for (int i = 1; i < 16; i++) Xb[s0 + i][threadIdx.x] = x[i];
+    }
+    __syncthreads();
+    // rows s0 + 16 .. 63, 3 (2, 1) a thread, 4 columns each
+    float4 acc[3];
+    const int n = (MX_NB - 16 - s0) / 16;
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      if (i < n) acc[i] = *reinterpret_cast<const float4*>(&Xb[s0 + 16 + 16 * i + ty][4 * tx]);
+#pragma unroll 4
+    for (int m = 0; m < 16; m++) {
+      const float4 x = *reinterpret_cast<const float4*>(&Xb[s0 + m][4 * tx]);
+#pragma unroll
+      for (int i = 0; i < 3; i++)
+        if (i < n) {
+          const float l = Lt[s0 + m][s0 + 16 + 16 * i + ty];
+          acc[i].x = fmaf(-l, x.x, acc[i].x);
+          acc[i].y = fmaf(-l, x.y, acc[i].y);
+          acc[i].z = fmaf(-l, x.z, acc[i].z);
+          acc[i].w = fmaf(-l, x.w, acc[i].w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      if (i < n) *reinterpret_cast<float4*>(&Xb[s0 + 16 + 16 * i + ty][4 * tx]) = acc[i];
+    __syncthreads();
+  }
+}
+
+// X[64 (b + 1) + ...] -= L X_b for 16 NI rows below; thread (ty, tx): rows 4 ty + 64 i .. + 3, columns 4 tx .. + 3.
+template <int NI>
+__device__ __forceinline__ void row_block_update(RowBlockSmem& s, int b) {
+  const float(*L)[RB_LLD] = s.L[b & 1];
+  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+  const float(*Xb)[RB_COLS] = &s.X[MX_NB * b];
+  float(*Xr)[RB_COLS] = &s.X[MX_NB * (b + 1)];
+  float acc[NI][4][4];
+#pragma unroll
+  for (int i = 0; i < NI; i++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const float4 f = *reinterpret_cast<const float4*>(&Xr[64 * i + 4 * ty + q][4 * tx]);
+      acc[i][q][0] = f.x;
+      acc[i][q][1] = f.y;
+      acc[i][q][2] = f.z;
+      acc[i][q][3] = f.w;
+    }
+#pragma unroll 4
+  for (int m = 0; m < MX_NB; m++) {
+    const float4 x = *reinterpret_cast<const float4*>(&Xb[m][4 * tx]);
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const float4 l = *reinterpret_cast<const float4*>(&L[m][64 * i + 4 * ty]);
+      const float lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        acc[i][q][0] = fmaf(-lv[q], x.x, acc[i][q][0]);
+        acc[i][q][1] = fmaf(-lv[q], x.y, acc[i][q][1]);
+        acc[i][q][2] = fmaf(-lv[q], x.z, acc[i][q][2]);
+        acc[i][q][3] = fmaf(-lv[q], x.w, acc[i][q][3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NI; i++)
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+      *reinterpret_cast<float4*>(&Xr[64 * i + 4 * ty + q][4 * tx]) =
+          make_float4(acc[i][q][0], acc[i][q][1], acc[i][q][2], acc[i][q][3]);
+}
+
+__global__ void __launch_bounds__(RB_THREADS, 1)
+    k_row_block(float* __restrict__ A, int64_t lda, int64_t N, int64_t p0, const PanelScratch* __restrict__ scratch) {  // null: in A
+  extern __shared__ __align__(16) unsigned char rb_raw[];
+  RowBlockSmem& s = *reinterpret_cast<RowBlockSmem*>(rb_raw);
+  pdl_wait();
+  const int tid = threadIdx.x;
+  const int64_t pe = p0 + TC_PANEL, c0 = pe + blockIdx.x * (int64_t)RB_COLS;
+  const int cols = N - c0 < RB_COLS ? int(N - c0) : RB_COLS;
+  // the blocks of the panel's rows 64 b ..: its diagonal block's L, and the rows below
+  auto fetch = [&](int b) {
+    const int64_t k0 = p0 + MX_NB * b;
+    const int below = TC_PANEL - MX_NB * (b + 1);
+    const float* D = scratch ? &scratch[b].d[0][0] : A + k0 * lda + k0;
+    const int64_t ldd = scratch ? MX_NB : lda;
+    const int m = tid % MX_NB;
+    for (int i = tid / MX_NB; i < MX_NB; i += RB_THREADS / MX_NB) cp_async4(&s.Lt[b & 1][m][i], D + i * ldd + m, true);
+    for (int r = tid / MX_NB; r < below; r += RB_THREADS / MX_NB)
+      cp_async4(&s.L[b & 1][m][r], A + (k0 + MX_NB + r) * lda + k0 + m, true);
+  };
+  for (int e = tid; e < TC_PANEL * RB_COLS; e += RB_THREADS) {
+    const int r = e / RB_COLS, c = e % RB_COLS;
+    cp_async4(&s.X[r][c], c < cols ? A + (p0 + r) * lda + c0 + c : A, c < cols);
+  }
+  fetch(0);
+  for (int b = 0; b < TC_PANEL / MX_NB; b++) {
+    cp_async_all();
+    __syncthreads();
+    if (b + 1 < TC_PANEL / MX_NB) fetch(b + 1);
+    row_block_solve(&s.X[MX_NB * b], s.Lt[b & 1]);
+    if (b == 0)
+      row_block_update<3>(s, 0);
+    else if (b == 1)
+      row_block_update<2>(s, 1);
+    else if (b == 2)
+      row_block_update<1>(s, 2);
+    __syncthreads();
+  }
+  for (int e = tid; e < TC_PANEL * RB_COLS; e += RB_THREADS) {
+    const int r = e / RB_COLS, c = e % RB_COLS;
+    if (c < cols) A[(p0 + r) * lda + c0 + c] = s.X[r][c];
+  }
+  if (scratch) panel_store(A, lda, p0, pe, scratch);
 }
 
 // ---------------------------------------------------------------- tensor cores
@@ -940,18 +1272,40 @@ static int side_stream(SideStream*& out) {
   return OK;
 }
 
+static int64_t lu_tc_bytes(int64_t N) {
+  // two alternating split-operand buffers and the panel's scratch area
+  return 2 * round256(gemm_pre_bytes(N, N, TC_PANEL)) + round256(TC_PANEL / MX_NB * int64_t(sizeof(PanelScratch)));
+}
+
+static bool g_attr_panel[64];
+static int panel_attr() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return CUDA_ERR;
+  if (dev >= 0 && dev < 64 && g_attr_panel[dev]) return OK;
+  if (cudaFuncSetAttribute(k_panel_step, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(PanelSmem))) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_row_block, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(RowBlockSmem))) !=
+          cudaSuccess ||
+      cudaFuncSetAttribute(k_trsm_right_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM) != cudaSuccess ||
+      cudaFuncSetAttribute(k_trsm_left_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, TRSM_SMEM) != cudaSuccess)
+    return CUDA_ERR;
+  if (dev >= 0 && dev < 64) g_attr_panel[dev] = true;
+  return OK;
+}
+
 // FP32 LU without pivoting, two-level blocked: panels of 256 columns are
-// factored with the 64-wide kernels above (diagonal block, triangular
-// solves) and tensor-core updates (K = 64) inside the panel and its row
-// block; the trailing matrix is updated once per panel by the persistent
-// tensor-core GEMM (K = 256) from operands pre-split into `work`.  err
-// receives 1 if a tensor-core wait ran out.
-constexpr int TC_PANEL = 256;
+// factored by k_panel_step (tall ones by the separate kernels, with
+// tensor-core updates, K = 64), their row blocks by k_row_block; the trailing
+// matrix is updated once per panel by the persistent tensor-core GEMM (K =
+// 256) from operands pre-split into `work`.  err receives 1 if a tensor-core
+// wait ran out.
 static int lu_nopiv_f32_tc(float* A, int64_t lda, int64_t N, int* err, uint8_t* work, cudaStream_t s) {
   const int reserve = lookahead_reserve();
   SideStream* ss = nullptr;
   if (reserve > 0 && side_stream(ss) != OK) return CUDA_ERR;
-  if (gemm_pre_attr() != OK) return CUDA_ERR;
+  if (gemm_pre_attr() != OK || panel_attr() != OK) return CUDA_ERR;
+  PanelScratch* scratch =
+      reinterpret_cast<PanelScratch*>(work + 2 * round256(gemm_pre_bytes(N, N, TC_PANEL)));
   // With lookahead the trailing update of panel p runs in three parts: the
   // next panel's 256 columns first, on every SM, on the caller's stream;
   // then, on the side stream with all but `reserve` SMs, the remaining
@@ -965,15 +1319,25 @@ static int lu_nopiv_f32_tc(float* A, int64_t lda, int64_t N, int* err, uint8_t* 
   int buf = 0;
   for (int64_t p0 = 0; p0 < N; p0 += TC_PANEL) {
     const int64_t pe = p0 + TC_PANEL < N ? p0 + TC_PANEL : N;
+    // one launch a step while its CTAs all fit on the SMs that the default
+    // lookahead leaves free (whatever it is set to: the factors are the same
+    // bit for bit either way)
+    const bool fused = (N - p0 + PS_ROWS - 1) / PS_ROWS <= num_sms() / 5;
     for (int64_t k0 = p0; k0 < pe; k0 += MX_NB) {
       const int nb = pe - k0 < MX_NB ? int(pe - k0) : MX_NB;
-      pdl_launch(k_diag_lu_f32, dim3(1), dim3(256), 0, s, A, lda, k0, nb);
       const int64_t below = N - k0 - nb, right = pe - k0 - nb;
+      const unsigned g = below > 0 ? unsigned((below + PS_ROWS - 1) / PS_ROWS) : 1u;
+      if (fused) {
+        pdl_launch(k_panel_step, dim3(g), dim3(PS_THREADS), sizeof(PanelSmem), s, A, lda, N, k0, nb, pe,
+                   scratch + (k0 - p0) / MX_NB);
+        continue;
+      }
+      pdl_launch(k_diag_lu_f32, dim3(1), dim3(256), 0, s, A, lda, k0, nb);
       if (below > 0)
-        pdl_launch(k_trsm_right_f32, dim3(unsigned((below + TRSM_COLS - 1) / TRSM_COLS)), dim3(TRSM_COLS), 0, s, A,
-                   lda, k0 + nb, N, k0, nb);
+        pdl_launch(k_trsm_right_f32, dim3(unsigned((below + TRSM_COLS - 1) / TRSM_COLS)), dim3(TRSM_COLS), TRSM_SMEM, s,
+                   A, lda, k0 + nb, N, k0, nb);
       if (right > 0) {
-        pdl_launch(k_trsm_left_f32, dim3(unsigned((right + TRSM_COLS - 1) / TRSM_COLS)), dim3(TRSM_COLS), 0, s, A,
+        pdl_launch(k_trsm_left_f32, dim3(unsigned((right + TRSM_COLS - 1) / TRSM_COLS)), dim3(TRSM_COLS), TRSM_SMEM, s, A,
                    lda, k0 + nb, pe, k0, nb);
         const int st = gemm_sub_tf32x3(A + (k0 + nb) * lda + k0 + nb, lda, A + (k0 + nb) * lda + k0, lda,
                                        A + k0 * lda + k0 + nb, lda, below, right, nb, err, s);
@@ -981,23 +1345,16 @@ static int lu_nopiv_f32_tc(float* A, int64_t lda, int64_t N, int* err, uint8_t* 
       }
     }
     const int64_t rest = N - pe;
-    if (rest <= 0) break;
+    if (rest <= 0) {
+      if (fused) pdl_launch(k_panel_store, dim3(32), dim3(256), 0, s, A, lda, p0, pe, scratch);
+      break;
+    }
     if (top_pending) {  // the row block reads the columns `top` updates
       if (cudaStreamWaitEvent(s, ss->top, 0) != cudaSuccess) return CUDA_ERR;
       top_pending = false;
     }
-    // row block right of the panel: U12 = L11^-1 A12, 64 rows at a time
-    for (int64_t k0 = p0; k0 < pe; k0 += MX_NB) {
-      const int nb = pe - k0 < MX_NB ? int(pe - k0) : MX_NB;
-      pdl_launch(k_trsm_left_f32, dim3(unsigned((rest + TRSM_COLS - 1) / TRSM_COLS)), dim3(TRSM_COLS), 0, s, A, lda,
-                 pe, N, k0, nb);
-      const int64_t rows = pe - k0 - nb;
-      if (rows > 0) {
-        const int st = gemm_sub_tf32x3(A + (k0 + nb) * lda + pe, lda, A + (k0 + nb) * lda + k0, lda, A + k0 * lda + pe,
-                                       lda, rows, rest, nb, err, s);
-        if (st != OK) return st;
-      }
-    }
+    pdl_launch(k_row_block, dim3(unsigned((rest + RB_COLS - 1) / RB_COLS)), dim3(RB_THREADS), sizeof(RowBlockSmem), s, A,
+               lda, N, p0, fused ? scratch : nullptr);
     const int K = int(pe - p0);
     float* C = A + pe * lda + pe;
     uint8_t* w = work + (ss ? buf * buf_bytes : 0);
@@ -1095,13 +1452,13 @@ __global__ void k_col_scale(const unsigned long long* __restrict__ maxbits, doub
 constexpr int SC_COLS = 512;
 __global__ void __launch_bounds__(256) k_scale_to_f32(const double* __restrict__ A, int64_t lda,
                                                       const double* __restrict__ c, float* __restrict__ S,
-                                                      int64_t N) {
+                                                      int64_t lds, int64_t N) {
   const int64_t chunks = (N + SC_COLS - 1) / SC_COLS;
   const int64_t i = blockIdx.x / chunks, j = (blockIdx.x % chunks) * SC_COLS + 2 * threadIdx.x;
   if (i >= N || j >= N) return;
   const double* a = A + i * lda + j;
-  float* o = S + i * N + j;
-  if (j + 1 < N && (lda % 2) == 0 && (N % 2) == 0 && (reinterpret_cast<uintptr_t>(A) % 16) == 0) {
+  float* o = S + i * lds + j;
+  if (j + 1 < N && (lda % 2) == 0 && (lds % 2) == 0 && (reinterpret_cast<uintptr_t>(A) % 16) == 0) {
     const double2 v = *reinterpret_cast<const double2*>(a);
     const double2 cc = *reinterpret_cast<const double2*>(c + j);
     *reinterpret_cast<float2*>(o) = make_float2(float(v.x * cc.x), float(v.y * cc.y));
@@ -1279,20 +1636,24 @@ __device__ __forceinline__ bool wait_flag(const int* flags, int j, int epoch, in
   return true;
 }
 
-// For row block b of the unit lower (LOWER) or upper triangle of LU:
-// Dinv[b] = T_bb^-1 and Mla[b] = T_bb^-1 T_bg (g = b - 1 / b + 1; zero when
-// b has no such neighbour), both 64 x 64 FP64 stored column-major
-// (element (i, m) at m * 64 + i); rows / columns beyond N are the identity
-// in T_bb and zero in T_bg.  One CTA of 64 threads per block, one column per
-// thread.
+// For row block b of the unit lower (grid row 0) and upper (grid row 1)
+// triangle of LU: Dinv[b] = T_bb^-1 and Mla[b] = T_bb^-1 T_bg (g = b - 1 /
+// b + 1; zero when b has no such neighbour), both 64 x 64 FP64 stored
+// column-major (element (i, m) at m * 64 + i); rows / columns beyond N are the
+// identity in T_bb and zero in T_bg.  256 threads per block: thread (k, g)
+// holds rows g, g + 4, ... of column k and takes each finished row off the
+// others as it comes (64 short steps; one thread per column summing its own
+// dot products took 70 to 85 us per triangle, whatever N).
 template <bool LOWER>
-__global__ void __launch_bounds__(TS_B) k_diag_inverse(const float* __restrict__ LU, int64_t lda, int64_t N,
-                                                      double* __restrict__ Dinv, double* __restrict__ Mla) {
-  __shared__ float T[TS_B][TS_B];    // the factor block (FP32 values, exact)
-  __shared__ double Xc[TS_B][TS_B];  // Xc[row][col]; thread k owns column k
+__device__ __forceinline__ void diag_inverse(const float* __restrict__ LU, int64_t lda, int64_t N,
+                                             double* __restrict__ Dinv, double* __restrict__ Mla, float (*T)[TS_B],
+                                             double (*Xc)[TS_B + 1]) {
   const int nblk = int((N + TS_B - 1) / TS_B);
   const int64_t b0 = (int64_t)blockIdx.x * TS_B;
   const int nb = N - b0 < TS_B ? int(N - b0) : TS_B;
+  const int k = threadIdx.x % TS_B, grp = threadIdx.x / TS_B;
+  double* row = &Xc[0][0];  // [2][64] finished rows, then the reciprocal pivots; the matrix itself later
+  double* piv = row + 2 * TS_B;
   for (int e = threadIdx.x; e < TS_B * TS_B; e += blockDim.x) {
     const int i = e / TS_B, j = e % TS_B;
     float v = (i == j) ? 1.f : 0.f;
@@ -1303,20 +1664,30 @@ __global__ void __launch_bounds__(TS_B) k_diag_inverse(const float* __restrict__
     T[i][j] = v;
   }
   __syncthreads();
-  const int k = threadIdx.x;  // column k of the inverse: T x = e_k
-  if (LOWER) {
-    for (int i = 0; i < TS_B; i++) {
-      double v = (i == k) ? 1.0 : 0.0;
-      for (int m = 0; m < i; m++) v = fma(-double(T[i][m]), Xc[m][k], v);
-      Xc[i][k] = v;
+  if (!LOWER && threadIdx.x < TS_B) piv[threadIdx.x] = 1.0 / double(T[threadIdx.x][threadIdx.x]);
+  __syncthreads();
+  double x[TS_B / 4];  // rows grp + 4 q of column k of the inverse
+#pragma unroll
+  for (int q = 0; q < TS_B / 4; q++) x[q] = grp + 4 * q == k ? 1.0 : 0.0;
+#pragma unroll
+  for (int st = 0; st < TS_B; st++) {
+    const int i = LOWER ? st : TS_B - 1 - st;
+    if (grp == (i & 3)) {
+      if (!LOWER) x[i >> 2] *= piv[i];
+      row[(st & 1) * TS_B + k] = x[i >> 2];
     }
-  } else {
-    for (int i = TS_B - 1; i >= 0; i--) {
-      double v = (i == k) ? 1.0 : 0.0;
-      for (int m = i + 1; m < TS_B; m++) v = fma(-double(T[i][m]), Xc[m][k], v);
-      Xc[i][k] = v / double(T[i][i]);
+    __syncthreads();
+    const double xi = row[(st & 1) * TS_B + k];
+#pragma unroll
+    for (int q = 0; q < TS_B / 4; q++) {
+      const int m = grp + 4 * q;
+      if (LOWER ? 4 * q + 3 > i : 4 * q < i)
+        if (LOWER ? m > i : m < i) x[q] = fma(-double(T[m][i]), xi, x[q]);
     }
   }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < TS_B / 4; q++) Xc[grp + 4 * q][k] = x[q];
   __syncthreads();
   double* D = Dinv + (int64_t)blockIdx.x * TS_B * TS_B;
   for (int e = threadIdx.x; e < TS_B * TS_B; e += blockDim.x) D[e] = Xc[e % TS_B][e / TS_B];
@@ -1333,15 +1704,35 @@ __global__ void __launch_bounds__(TS_B) k_diag_inverse(const float* __restrict__
     T[i][j] = (i < nb && g0 + j < N) ? LU[(b0 + i) * lda + g0 + j] : 0.f;
   }
   __syncthreads();
-  for (int i = 0; i < TS_B; i++) {
-    double v0 = 0.0, v1 = 0.0;
-#pragma unroll 8
-    for (int m = 0; m < TS_B; m += 2) {
-      v0 = fma(Xc[i][m], double(T[m][k]), v0);
-      v1 = fma(Xc[i][m + 1], double(T[m + 1][k]), v1);
-    }
-    Mo[(int64_t)k * TS_B + i] = v0 + v1;
+#pragma unroll
+  for (int q = 0; q < TS_B / 4; q++) x[q] = 0.0;
+#pragma unroll 4
+  for (int m = 0; m < TS_B; m++) {
+    const double t = double(T[m][k]);
+#pragma unroll
+    for (int q = 0; q < TS_B / 4; q++) x[q] = fma(Xc[grp + 4 * q][m], t, x[q]);
   }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < TS_B / 4; q++) Xc[grp + 4 * q][k] = x[q];
+  __syncthreads();
+  for (int e = threadIdx.x; e < TS_B * TS_B; e += blockDim.x) Mo[e] = Xc[e % TS_B][e / TS_B];
+}
+
+struct DiagInverseSmem {
+  float T[TS_B][TS_B];            // the factor block (FP32 values, exact)
+  double Xc[TS_B][TS_B + 1];      // Xc[row][col]
+};
+
+__global__ void __launch_bounds__(256) k_diag_inverse(const float* __restrict__ LU, int64_t lda, int64_t N,
+                                                      double* __restrict__ dinv_l, double* __restrict__ mla_l,
+                                                      double* __restrict__ dinv_u, double* __restrict__ mla_u) {
+  extern __shared__ __align__(16) unsigned char di_raw[];
+  DiagInverseSmem& s = *reinterpret_cast<DiagInverseSmem*>(di_raw);
+  if (blockIdx.y == 0)
+    diag_inverse<true>(LU, lda, N, dinv_l, mla_l, s.T, s.Xc);
+  else
+    diag_inverse<false>(LU, lda, N, dinv_u, mla_u, s.T, s.Xc);
 }
 
 // X (nrhs x N, row r at X + r N) <- T^-1 X with T the unit lower (LOWER) or
@@ -1610,7 +2001,7 @@ extern "C" int64_t tb_gemm_tf32x3_workspace(int64_t M, int64_t N, int64_t K) {
 
 extern "C" int64_t tb_lu_nopiv_f32_tc_workspace(int64_t N) {
   if (N <= 0) return 0;
-  return 2 * round256(gemm_pre_bytes(N, N, TC_PANEL));  // two alternating split-operand buffers
+  return lu_tc_bytes(N);
 }
 
 extern "C" int tb_lu_nopiv_f32_tc(float* A, int64_t lda, int64_t N, void* work, int64_t work_bytes, int* err,
@@ -1636,13 +2027,18 @@ extern "C" int tb_gemm_sub_tf32x3(float* C, int64_t ldc, const float* A, int64_t
   return gemm_sub_tf32x3(C, ldc, A, lda, B, ldb, M, N, int(K), err, (cudaStream_t)stream);
 }
 
+// Row stride of the FP32 factors: rows start at 16-byte boundaries whatever N,
+// which the update's and the sweeps' vector accesses need (2,501 elements: the
+// updates take 0.9 instead of 1.1 ms).
+static int64_t factor_stride(int64_t N) { return (N + 3) / 4 * 4; }
+
 extern "C" int64_t tb_solve_mixed_workspace(int64_t N, int64_t nrhs) {
   if (N <= 0 || nrhs <= 0) return 0;
   const int64_t nblk = (N + TS_B - 1) / TS_B;
   // FP32 factors, column scales, correction / residual block, the forward
   // sweep's output, 2 * nrhs maxima, inverses of the diagonal blocks of both
   // factors and their lookahead products, sweep flags and the error word
-  return round256(N * N * 4) + round256(N * 8) + 2 * round256(nrhs * N * 8) + 256 +
+  return round256(N * factor_stride(N) * 4) + round256(N * 8) + 2 * round256(nrhs * N * 8) + 256 +
          4 * round256(nblk * TS_B * TS_B * 8) + round256((nblk + 1) * 4) + 256 +
          round256(tb_lu_nopiv_f32_tc_workspace(N));
 }
@@ -1656,8 +2052,9 @@ extern "C" int tb_solve_mixed(const double* A, int64_t lda, int64_t N, const dou
   cudaStream_t s = (cudaStream_t)stream;
   char* w = static_cast<char*>(work);
   const int64_t nblk = (N + TS_B - 1) / TS_B;
+  const int64_t lds = factor_stride(N);
   float* S = reinterpret_cast<float*>(w);
-  w += round256(N * N * 4);
+  w += round256(N * lds * 4);
   double* c = reinterpret_cast<double*>(w);
   w += round256(N * 8);
   double* D = reinterpret_cast<double*>(w);
@@ -1687,13 +2084,15 @@ extern "C" int tb_solve_mixed(const double* A, int64_t lda, int64_t N, const dou
   k_col_scale<<<unsigned((N + 255) / 256), 256, 0, s>>>(maxbits, c, N);
   {
     const int64_t chunks = (N + SC_COLS - 1) / SC_COLS;
-    k_scale_to_f32<<<unsigned(N * chunks), SC_COLS / 2, 0, s>>>(A, lda, c, S, N);
+    k_scale_to_f32<<<unsigned(N * chunks), SC_COLS / 2, 0, s>>>(A, lda, c, S, lds, N);
   }
   if (cudaMemsetAsync(err, 0, sizeof(int), s) != cudaSuccess) return CUDA_ERR;
-  int st = lu_nopiv_f32_tc(S, N, N, err, gemm_work, s);
+  int st = lu_nopiv_f32_tc(S, lds, N, err, gemm_work, s);
   if (st != OK) return st;
-  k_diag_inverse<true><<<unsigned(nblk), TS_B, 0, s>>>(S, N, N, dinv_l, mla_l);
-  k_diag_inverse<false><<<unsigned(nblk), TS_B, 0, s>>>(S, N, N, dinv_u, mla_u);
+  if (cudaFuncSetAttribute(k_diag_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(DiagInverseSmem))) !=
+      cudaSuccess)
+    return CUDA_ERR;
+  k_diag_inverse<<<dim3(unsigned(nblk), 2), 256, sizeof(DiagInverseSmem), s>>>(S, lds, N, dinv_l, mla_l, dinv_u, mla_u);
   if (cudaMemsetAsync(flags, 0, sizeof(int) * (nblk + 1), s) != cudaSuccess) return CUDA_ERR;
   constexpr int SW8 = sweep_dyn_bytes<8>(), SW16 = sweep_dyn_bytes<16>();
   if (cudaFuncSetAttribute(k_residual<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, residual_smem<4>()) !=
@@ -1734,17 +2133,17 @@ extern "C" int tb_solve_mixed(const double* A, int64_t lda, int64_t N, const dou
     const size_t vec_bytes = sizeof(double) * N * nrhs;
     if (cudaMemsetAsync(Y, 0xff, vec_bytes, s) != cudaSuccess) return CUDA_ERR;
     if (nr <= 8)
-      k_trsv_sweep<true, 8><<<unsigned(nblk), 256, SW8, s>>>(S, N, N, dinv_l, mla_l, D, Y, nr, flags, ++epoch, err,
+      k_trsv_sweep<true, 8><<<unsigned(nblk), 256, SW8, s>>>(S, lds, N, dinv_l, mla_l, D, Y, nr, flags, ++epoch, err,
                                                                   wcyc);
     else
-      k_trsv_sweep<true, 16><<<unsigned(nblk), 256, SW16, s>>>(S, N, N, dinv_l, mla_l, D, Y, nr, flags, ++epoch, err,
+      k_trsv_sweep<true, 16><<<unsigned(nblk), 256, SW16, s>>>(S, lds, N, dinv_l, mla_l, D, Y, nr, flags, ++epoch, err,
                                                                    wcyc);
     if (cudaMemsetAsync(D, 0xff, vec_bytes, s) != cudaSuccess) return CUDA_ERR;
     if (nr <= 8)
-      k_trsv_sweep<false, 8><<<unsigned(nblk), 256, SW8, s>>>(S, N, N, dinv_u, mla_u, Y, D, nr, flags, ++epoch, err,
+      k_trsv_sweep<false, 8><<<unsigned(nblk), 256, SW8, s>>>(S, lds, N, dinv_u, mla_u, Y, D, nr, flags, ++epoch, err,
                                                                    wcyc);
     else
-      k_trsv_sweep<false, 16><<<unsigned(nblk), 256, SW16, s>>>(S, N, N, dinv_u, mla_u, Y, D, nr, flags, ++epoch,
+      k_trsv_sweep<false, 16><<<unsigned(nblk), 256, SW16, s>>>(S, lds, N, dinv_u, mla_u, Y, D, nr, flags, ++epoch,
                                                                     err, wcyc);
     if (cudaMemsetAsync(maxes, 0, sizeof(unsigned long long) * 2 * nr, s) != cudaSuccess) return CUDA_ERR;
     {
