@@ -588,13 +588,33 @@ struct AxialField {
 
 // One thread per particle: the stage loop fully unrolled, so the six stage
 // vectors stay in registers (the team tracers share theirs in shared memory).
-__global__ void __launch_bounds__(128) k_trace_axial(TraceParams P) {
+// The kernel is bound by the latency of a particle's own chain (1.6 us an
+// evaluation, alone or among others), so what counts is that all particles
+// are under way at once: with BLOCKS = 3 blocks a SM the registers hold
+// everything (168 each; 727 us for one electron, 877 with 4), with 4 the last
+// quarter of a larger beam need not wait for a second round (65,537 electrons:
+// 2.3 instead of 2.9 ms).  Reading a warp's table rows together through shared
+// memory costs more than it saves (3.0 ms).
+template <int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_trace_axial(TraceParams P) {
   AxialField field{P};
   for (;;) {
     int64_t idx = atomicAdd(P.work, 1);
     if (idx >= P.n) break;
     rk45_particle<AxialField, true>(P, idx, field, nullptr, true);
   }
+}
+
+template <int BLOCKS>
+static int launch_axial(const TraceParams& P, cudaStream_t s) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_axial<BLOCKS>, 128, 0) != cudaSuccess || per_sm < 1)
+    per_sm = 1;
+  int64_t blocks = (int64_t)num_sms() * per_sm;
+  const int64_t by_work = (P.n + 127) / 128;
+  if (blocks > by_work) blocks = by_work;
+  k_trace_axial<BLOCKS><<<unsigned(blocks), 128, 0, s>>>(P);
+  return launch_status();
 }
 
 template <int TW, bool GEOM, int MODE>
@@ -1661,16 +1681,7 @@ static int trace_rk45(const double* start, const double* t0, const double* qm, c
   }
   cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemsetAsync(work, 0, sizeof(int32_t), s) != cudaSuccess) return CUDA_ERR;
-  if (axial) {
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trace_axial, 128, 0) != cudaSuccess || per_sm < 1)
-      per_sm = 1;
-    int64_t blocks = (int64_t)num_sms() * per_sm;
-    int64_t by_work = (n + 127) / 128;
-    if (blocks > by_work) blocks = by_work;
-    k_trace_axial<<<unsigned(blocks), 128, 0, s>>>(P);
-    return launch_status();
-  }
+  if (axial) return n <= (int64_t)num_sms() * 3 * 128 ? launch_axial<3>(P, s) : launch_axial<4>(P, s);
   int tw = opts->team_warps;
   if (tw == 0) {
     // Fill the GPU: about 32 resident warps per SM.
