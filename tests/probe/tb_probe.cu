@@ -38,14 +38,39 @@ __global__ void k_probe_math(const double* __restrict__ x, int64_t n, int fn, do
     case 2: r = log_bf(v); break;
     case 3: r = rsqrt_h3(v); break;
     case 4: r = neglog_tab(v); break;
+    case 5: r = div_by(v, 0.00075, 1.0 / 0.00075); break;
+    case 6: r = div_by(v, 9.0, 1.0 / 9.0); break;
     case 10: r = 1.0 / v; break;
     case 11: r = 1.0 / sqrt(v); break;
+    case 13: r = v / 0.00075; break;
+    case 14: r = v / 9.0; break;
     default: r = log(v); break;
   }
   out[i] = r;
 }
 
+// Derivatives 1..8 of an axial table at z (NaN outside it); wide: the grid's
+// constants and the 32-byte reads.
+__global__ void k_probe_axial(const double* __restrict__ z, int64_t n, const double* zi, const double* coeff,
+                              int64_t Nz, int wide, double* __restrict__ out) {
+  __shared__ double grid[4];
+  if (threadIdx.x == 0) axial_grid(zi, Nz, grid);
+  __syncthreads();
+  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double d[NDERIV];
+  const bool in = wide ? axial_eval(z[i], zi, coeff, Nz, d, 1, grid, true) : axial_eval(z[i], zi, coeff, Nz, d, 1);
+  for (int k = 1; k < NDERIV; k++) out[i * (NDERIV - 1) + k - 1] = in ? d[k] : __longlong_as_double(0x7ff8000000000000LL);
+}
+
 }  // namespace tb
+
+extern "C" int tb_probe_axial(const double* z, int64_t n, const double* zi, const double* coeff, int64_t Nz, int wide,
+                              double* out, tb_probe_stream_t stream) {
+  if (n <= 0 || !z || !zi || !coeff || Nz < 2 || !out) return tb::BAD_ARG;
+  tb::k_probe_axial<<<unsigned((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(z, n, zi, coeff, Nz, wide, out);
+  return tb::launch_status();
+}
 
 extern "C" int tb_probe_math(const double* x, int64_t n, int fn, double* out, tb_probe_stream_t stream) {
   if (n < 0 || (n > 0 && (!x || !out))) return tb::BAD_ARG;

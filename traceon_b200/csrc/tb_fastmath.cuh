@@ -76,6 +76,15 @@ __device__ __forceinline__ double rsqrt_h3(double x) {
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// a / b from y = 1 / b rounded to nearest: the product, its exact remainder by
+// a fused multiply-add, and one correction (P. Markstein, IBM J. Res. Dev. 34,
+// 1990: the rounded quotient).  For divisors that stay the same over a launch:
+// three dependent operations instead of a division.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
+
 // Coefficients 1/(2j+1), j = 1..10, of the atanh series.
 __constant__ double C_ATANH[10] = {1.0 / 3,  1.0 / 5,  1.0 / 7,  1.0 / 9,  1.0 / 11,
                                    1.0 / 13, 1.0 / 15, 1.0 / 17, 1.0 / 19, 1.0 / 21};

@@ -74,17 +74,66 @@ inline int num_sms() {
 // touch 32 lines each and are bound by the L1's tag lookups, not by bytes:
 // a row's six coefficients are read as three pairs (rows start at multiples
 // of 48 bytes; a table that is not 16-byte aligned takes single loads).
+// Without derivative 0 (the field) a row's other 384 bytes are read 32 at a
+// time: eleven loads at the 32-byte boundaries inside and two of 16 bytes,
+// 13 lookups a lane instead of 24.  Rows start at multiples of 432 bytes, so
+// the boundary lies at the first byte or 16 behind it, row by row, and a
+// select puts the pairs in place.
+//
+// grid: on the device, {z_0, z_last, dz, 1 / dz} where a kernel has them at
+// hand (axial_grid), or null.
 __host__ __device__ inline bool axial_eval(double z, const double* zi, const double* coeff, int64_t Nz,
-                                           double* d, int first = 0) {
+                                           double* d, int first = 0, const double* grid = nullptr,
+                                           bool wide = false) {
+#ifdef __CUDA_ARCH__
+  const double z0 = grid ? grid[0] : zi[0], zl = grid ? grid[1] : zi[Nz - 1];
+  if (!(z0 <= z && z <= zl)) return false;
+  int64_t idx = grid ? (int64_t)div_by(z - z0, grid[2], grid[3]) : (int64_t)((z - z0) / (zi[1] - zi[0]));
+#else
+  (void)grid;
   double z0 = zi[0], zl = zi[Nz - 1];
   if (!(z0 <= z && z <= zl)) return false;
   double dz = zi[1] - zi[0];
   int64_t idx = (int64_t)((z - z0) / dz);
+#endif
   if (idx < 0) idx = 0;
   if (idx > Nz - 2) idx = Nz - 2;
   double x = z - zi[idx];
   const double* C = coeff + idx * NDERIV * 6;
 #ifdef __CUDA_ARCH__
+  if (wide && first == 1 && (reinterpret_cast<uintptr_t>(coeff) & 15) == 0) {
+    const double2* row = reinterpret_cast<const double2*>(C + 6);  // 24 pairs
+    const bool odd = reinterpret_cast<uintptr_t>(row) & 16;        // the boundary is behind the first pair
+    const double2* quad = row + (odd ? 1 : 0);
+    double2 prev = odd ? row[0] : row[22];  // the pair that the eleven loads leave out beside the last
+    const double2 head = prev, last = row[23];
+    double2 c[3];
+    int have = 0, i = 1;
+#pragma unroll
+    for (int k = 0; k < 12; k++) {
+      double2 lo, hi;
+      if (k < 11) {
+        asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];"
+                     : "=d"(lo.x), "=d"(lo.y), "=d"(hi.x), "=d"(hi.y)
+                     : "l"(quad + 2 * k));
+      } else {
+        lo = head;
+        hi = last;
+      }
+      const double2 even_pair{odd ? prev.x : lo.x, odd ? prev.y : lo.y};
+      const double2 odd_pair = k < 11 ? double2{odd ? lo.x : hi.x, odd ? lo.y : hi.y} : last;
+      prev = hi;
+#pragma unroll
+      for (int w = 0; w < 2; w++) {
+        c[have++] = w == 0 ? even_pair : odd_pair;
+        if (have == 3) {
+          d[i++] = ((((c[0].x * x + c[0].y) * x + c[1].x) * x + c[1].y) * x + c[2].x) * x + c[2].y;
+          have = 0;
+        }
+      }
+    }
+    return true;
+  }
   if ((reinterpret_cast<uintptr_t>(coeff) & 15) == 0) {
 #pragma unroll
     for (int i = 0; i < NDERIV; i++) {
@@ -105,16 +154,32 @@ __host__ __device__ inline bool axial_eval(double z, const double* zi, const dou
   return true;
 }
 
+// The grid's constants for axial_eval.
+__device__ __forceinline__ void axial_grid(const double* zi, int64_t Nz, double* grid) {
+  grid[0] = zi[0];
+  grid[1] = zi[Nz - 1];
+  grid[2] = zi[1] - zi[0];
+  grid[3] = 1.0 / grid[2];
+}
+
 // potential_radial_derivs, radial.c:340-343
 __host__ __device__ inline double axial_potential(const double* d, double r2) {
   return d[0] - r2 / 4 * d[2] + r2 * r2 / 64. * d[4] - r2 * r2 * r2 / 2304. * d[6] +
          r2 * r2 * r2 * r2 / 147456. * d[8];
 }
 
-// field_radial_derivs, radial.c:376-383
+// field_radial_derivs, radial.c:376-383 (192 = 64 x 3, 9216 = 1024 x 9, 2304 =
+// 256 x 9: on the device the quotients by 3 and 9 in three operations each)
 __host__ __device__ inline void axial_field(const double* d, const double* p, double r2, double* f) {
+#ifdef __CUDA_ARCH__
+  const double r4 = r2 * r2;
+  const double t3 = div_by(r4, 3.0, 1.0 / 3.0), t9 = div_by(r4 * r2, 9.0, 1.0 / 9.0);
+  double fr = 0.5 * (d[2] - r2 / 8 * d[4] + t3 / 64 * d[6] - t9 / 1024 * d[8]);
+  double fz = -d[1] + r2 / 4 * d[3] - r4 / 64 * d[5] + t9 / 256 * d[7];
+#else
   double fr = 0.5 * (d[2] - r2 / 8 * d[4] + r2 * r2 / 192 * d[6] - r2 * r2 * r2 / 9216 * d[8]);
   double fz = -d[1] + r2 / 4 * d[3] - r2 * r2 / 64 * d[5] + r2 * r2 * r2 / 2304 * d[7];
+#endif
   f[0] = p[0] * fr;
   f[1] = p[1] * fr;
   f[2] = fz;

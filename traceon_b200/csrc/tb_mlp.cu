@@ -297,7 +297,7 @@ extern "C" int tb_mlp_adam(float* p, const float* g, float* m, float* v, void* p
 extern "C" int tb_mlp_features(const double* points, int64_t M, double r_max, double z_c, double z_half, void* X,
                                tb_stream_t stream) {
   if (M <= 0 || !points || !X || !(r_max > 0) || !(z_half > 0)) return BAD_ARG;
-  MlpDomain d{r_max, z_c, z_half};
+  const MlpDomain d = mlp_domain(r_max, z_c, z_half);
   k_features<<<unsigned((M + 255) / 256), 256, 0, (cudaStream_t)stream>>>(points, M, d,
                                                                           static_cast<__nv_bfloat16*>(X));
   return launch_status();

@@ -8,6 +8,8 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "tb_fastmath.cuh"
+
 namespace tb {
 
 constexpr int MLP_IN = 16;
@@ -36,7 +38,11 @@ constexpr int64_t MLP_NPARAM = MLP_OFF_B5 + MLP_OUT;
 // Normalisation of the inputs: rho = r / r_max, zeta = (z - z_c) / z_half.
 struct MlpDomain {
   double r_max, z_c, z_half;
+  double inv_r, inv_z;  // 1 / r_max, 1 / z_half, rounded (div_by)
 };
+inline MlpDomain mlp_domain(double r_max, double z_c, double z_half) {
+  return MlpDomain{r_max, z_c, z_half, 1.0 / r_max, 1.0 / z_half};
+}
 
 // SiLU through a single hardware tanh: silu(z) = z sigmoid(z) = h + h tanh(h)
 // with h = z / 2, in FP32 (tanh.approx.f32, one MUFU operation; maximum
@@ -88,7 +94,7 @@ __device__ __forceinline__ float silu_grad(float z) {
 // field is even in r) and five Fourier pairs in zeta, sin/cos(k pi zeta) for
 // k = 1..5, the higher harmonics by the angle-addition recurrence.
 __device__ __forceinline__ void mlp_features(double r, double z, const MlpDomain& d, float* f) {
-  float rho = float(r / d.r_max), zeta = float((z - d.z_c) / d.z_half);
+  float rho = float(div_by(r, d.r_max, d.inv_r)), zeta = float(div_by(z - d.z_c, d.z_half, d.inv_z));
   float p = rho * rho;
   f[0] = p;
   f[1] = zeta;

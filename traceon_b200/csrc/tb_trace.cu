@@ -572,14 +572,15 @@ __global__ void __launch_bounds__(TRACE_THREADS, 2) k_trace_bem(TraceParams P) {
 // Axial-interpolated field (field_radial_derivs_traceable): per thread.
 struct AxialField {
   const TraceParams& P;
+  const double* grid;  // axial_grid
   __device__ void operator()(const double* p, double* E, double* H) {
     double d[NDERIV];
     double r2 = p[0] * p[0] + p[1] * p[1];
-    if (axial_eval(p[2], P.az, P.aec, P.anz, d, 1))
+    if (axial_eval(p[2], P.az, P.aec, P.anz, d, 1, grid))
       axial_field(d, p, r2, E);
     else
       E[0] = E[1] = E[2] = 0.0;
-    if (P.amc && axial_eval(p[2], P.az, P.amc, P.anz, d, 1))
+    if (P.amc && axial_eval(p[2], P.az, P.amc, P.anz, d, 1, grid))
       axial_field(d, p, r2, H);
     else
       H[0] = H[1] = H[2] = 0.0;
@@ -588,16 +589,22 @@ struct AxialField {
 
 // One thread per particle: the stage loop fully unrolled, so the six stage
 // vectors stay in registers (the team tracers share theirs in shared memory).
-// The kernel is bound by the latency of a particle's own chain (1.6 us an
-// evaluation, alone or among others), so what counts is that all particles
-// are under way at once: with BLOCKS = 3 blocks a SM the registers hold
-// everything (168 each; 727 us for one electron, 877 with 4), with 4 the last
-// quarter of a larger beam need not wait for a second round (65,537 electrons:
-// 2.3 instead of 2.9 ms).  Reading a warp's table rows together through shared
-// memory costs more than it saves (3.0 ms).
+// The kernel is bound by the latency of a particle's own chain (1.5 us an
+// evaluation, alone or among others), so what counts is how many rounds the
+// beam takes: with BLOCKS = 3 blocks a SM the registers hold everything (168
+// each; a round takes 1.87 ms), with 4 a round holds a third more electrons and
+// takes 2.1 ms.  The dispatch picks the fewer rounds and 3 where they are equal
+// (65,537 electrons: 2.15 ms with 4, 2.50 with 3; 110,000: 3.98 and 3.74).
+// The grid's spacing divides by its reciprocal (axial_grid; 2.30 ms with
+// divisions).  Reading a warp's table rows together through shared memory costs
+// more than it saves (3.0 ms), and so do 32-byte reads with their selects (2.30
+// ms): unlike in the surrogate tracer the chain and not the L1 is the bound.
 template <int BLOCKS>
 __global__ void __launch_bounds__(128, BLOCKS) k_trace_axial(TraceParams P) {
-  AxialField field{P};
+  __shared__ double grid[4];
+  if (threadIdx.x == 0) axial_grid(P.az, P.anz, grid);
+  __syncthreads();
+  AxialField field{P, grid};
   for (;;) {
     int64_t idx = atomicAdd(P.work, 1);
     if (idx >= P.n) break;
@@ -684,6 +691,7 @@ struct SurrogateSmem {
   __nv_bfloat16 feat[SG_WARPS][32][MLP_LD_IN];
   float out[SG_WARPS][32][MLP_OUT];
   Seg segs[SG_MAX_SEGS];
+  double grid[4];  // axial_grid
 };
 
 __device__ inline void load_segments(Seg* seg, const double* __restrict__ segs, int nseg) {
@@ -802,11 +810,11 @@ __device__ __forceinline__ void bem_point_field(const TraceParams& P, const doub
 // Axial series of one coefficient table plus the learned correction
 // (cr, cz) times the envelope env: the radial part (cr rho^(p+1)) applied
 // as x * (F_r / r).
-__device__ __forceinline__ void axial_plus_correction(const TraceParams& P, const double* table, const double* p,
-                                                      double r2, double env_r, double env, float cr, float cz,
-                                                      double* F) {
+__device__ __forceinline__ void axial_plus_correction(const TraceParams& P, const double* grid, const double* table,
+                                                      const double* p, double r2, double env_r, double env, float cr,
+                                                      float cz, double* F) {
   double d[NDERIV];
-  if (table && axial_eval(p[2], P.az, table, P.anz, d, 1))
+  if (table && axial_eval(p[2], P.az, table, P.anz, d, 1, grid, true))
     axial_field(d, p, r2, F);
   else
     F[0] = F[1] = F[2] = 0.0;
@@ -837,17 +845,19 @@ __device__ __forceinline__ int surrogate_kind(const TraceParams& P, const Surrog
 }
 
 template <bool MAG>
-__device__ __forceinline__ void surrogate_apply(const TraceParams& P, const SurrogateParams& S, const double* p,
-                                                double r2, double r, const float* c, double* E, double* H);
+__device__ __forceinline__ void surrogate_apply(const TraceParams& P, const SurrogateParams& S, const double* grid,
+                                                const double* p, double r2, double r, const float* c, double* E,
+                                                double* H);
 
 template <bool MAG>
 __device__ __forceinline__ void surrogate_combine(const TraceParams& P, const SurrogateParams& S,
-                                                 const Seg* segs, const double* p, double r2, double r,
-                                                 bool live, const float* c, double* E, double* H, bool& used_bem) {
+                                                 const Seg* segs, const double* grid, const double* p, double r2,
+                                                 double r, bool live, const float* c, double* E, double* H,
+                                                 bool& used_bem) {
   const int kind = surrogate_kind(P, S, segs, p, r, live);
   used_bem = kind == FIELD_BEM;
   if (kind == FIELD_SURROGATE) {
-    surrogate_apply<MAG>(P, S, p, r2, r, c, E, H);
+    surrogate_apply<MAG>(P, S, grid, p, r2, r, c, E, H);
   } else if (kind == FIELD_BEM) {
     bem_point_field<MAG>(P, p, E, H);
   } else {
@@ -856,16 +866,21 @@ __device__ __forceinline__ void surrogate_combine(const TraceParams& P, const Su
   }
 }
 
-// Axial series + learned correction at p, inside the network's domain.
+// Axial series + learned correction at p, inside the network's domain.  The
+// threads' table rows are scattered, 24 reads of 16 bytes a row touch 32 lines
+// each, and twelve warps of them held the L1 for a quarter of the evaluation:
+// the 32-byte reads take the beam kernel (262,144 electrons) from 36.0 to 32.1
+// ms.  Divisors that a launch keeps divide by their reciprocals (div_by).
 template <bool MAG>
-__device__ __forceinline__ void surrogate_apply(const TraceParams& P, const SurrogateParams& S, const double* p,
-                                                double r2, double r, const float* c, double* E, double* H) {
-  const double rho = r / S.dom.r_max;
+__device__ __forceinline__ void surrogate_apply(const TraceParams& P, const SurrogateParams& S, const double* grid,
+                                                const double* p, double r2, double r, const float* c, double* E,
+                                                double* H) {
+  const double rho = div_by(r, S.dom.r_max, S.dom.inv_r);
   double env = 1.0;
   for (int i = 0; i < S.env_p; i++) env *= rho;
-  const double env_r = env / S.dom.r_max;
-  axial_plus_correction(P, P.aec, p, r2, env_r, env, c[0], c[1], E);
-  if (MAG) axial_plus_correction(P, P.amc, p, r2, env_r, env, c[2], c[3], H);
+  const double env_r = div_by(env, S.dom.r_max, S.dom.inv_r);
+  axial_plus_correction(P, grid, P.aec, p, r2, env_r, env, c[0], c[1], E);
+  if (MAG) axial_plus_correction(P, grid, P.amc, p, r2, env_r, env, c[2], c[3], H);
 }
 
 // The network's outputs y at a point contracted with the source strengths
@@ -897,7 +912,7 @@ __device__ void surrogate_field(const TraceParams& P, const SurrogateParams& S, 
   mlp_warp_forward(sm.mlp, sm.feat[warp], sm.out[warp]);
   float c[4];
   contract_outputs<MAG>(S, sm.out[warp][lane], c);
-  surrogate_combine<MAG>(P, S, sm.segs, p, r2, r, live, c, E, H, used_bem);
+  surrogate_combine<MAG>(P, S, sm.segs, sm.grid, p, r2, r, live, c, E, H, used_bem);
 }
 
 // The RKF45 particle loop of the surrogate tracer, shared by both network
@@ -1094,6 +1109,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1) k_trace_surrogate(TraceParams P
   SurrogateSmem& sm = *reinterpret_cast<SurrogateSmem*>(sg_raw);
   mlp_load_smem(sm.mlp, S.wb, S.pf);
   load_segments(sm.segs, S.segs, S.nseg);
+  if (threadIdx.x == 0) axial_grid(P.az, P.anz, sm.grid);
   __syncthreads();
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
 
@@ -1111,6 +1127,7 @@ __global__ void __launch_bounds__(SG_THREADS, 1)
   SurrogateSmem& sm = *reinterpret_cast<SurrogateSmem*>(sg_raw);
   mlp_load_smem(sm.mlp, S.wb, S.pf);
   load_segments(sm.segs, S.segs, S.nseg);
+  if (threadIdx.x == 0) axial_grid(P.az, P.anz, sm.grid);
   __syncthreads();
   const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
   for (int64_t base = (int64_t)blockIdx.x * SG_THREADS + warp * 32; base < M; base += (int64_t)gridDim.x * SG_THREADS) {
@@ -1159,6 +1176,7 @@ struct TcSmem {
   uint8_t act[TC_GROUPS][2][TC_ATOM];     // per group: activations, 128 rows x K <= 128
   float b1[MLP_H], bh[3][MLP_H], b5[MLP_OUT];
   Seg segs[SG_MAX_SEGS];
+  double grid[4];                         // axial_grid
   uint64_t mbar[TC_GROUPS];
   uint32_t tmem_base;
 };
@@ -1330,7 +1348,7 @@ struct TcEngine {
     const int kind = surrogate_kind(P, S, s.segs, p, r, live);
     used_bem = kind == FIELD_BEM;
     if (kind == FIELD_SURROGATE) {
-      surrogate_apply<MAG>(P, S, p, r2, r, c, E, H);
+      surrogate_apply<MAG>(P, S, s.grid, p, r2, r, c, E, H);
     } else {
       E[0] = E[1] = E[2] = 0.0;
       if (MAG) H[0] = H[1] = H[2] = 0.0;
@@ -1385,11 +1403,12 @@ struct TcEngine {
 // Shared set-up of the tcgen05 kernels: network and segments staged,
 // mbarriers initialised, TMEM allocated (warp 0).  Returns the aligned
 // shared-memory image.
-__device__ TcSmem& tc_setup(unsigned char* raw, const SurrogateParams& S) {
+__device__ TcSmem& tc_setup(unsigned char* raw, const TraceParams& P, const SurrogateParams& S) {
   const uint32_t a = tc::smem_u32(raw);
   TcSmem& s = *reinterpret_cast<TcSmem*>(raw + (((a + 1023u) & ~1023u) - a));
   tc_load_network(s, S.wb, S.pf);
   load_segments(s.segs, S.segs, S.nseg);
+  if (threadIdx.x == 32) axial_grid(P.az, P.anz, s.grid);
   if (threadIdx.x < TC_GROUPS) tc::mbar_init(&s.mbar[threadIdx.x], 1);
   if (threadIdx.x == 0) tc::fence_mbar_init();
   if (threadIdx.x / 32 == 0) {
@@ -1423,7 +1442,7 @@ __device__ __forceinline__ TcEngine<MAG> tc_engine(const TraceParams& P, const S
 template <bool MAG>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_trace_surrogate_tc(TraceParams P, SurrogateParams S) {
   extern __shared__ __align__(1024) unsigned char tc_raw[];
-  TcSmem& s = tc_setup(tc_raw, S);
+  TcSmem& s = tc_setup(tc_raw, P, S);
   TcEngine<MAG> eng = tc_engine<MAG>(P, S, s);
   surrogate_trace_loop<MAG>(P, S, eng);
   tc_teardown(s);
@@ -1437,7 +1456,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     k_surrogate_points_tc(TraceParams P, SurrogateParams S, const double* __restrict__ pts, int64_t M,
                           double* __restrict__ field, double* __restrict__ hfield, int32_t* __restrict__ used_bem) {
   extern __shared__ __align__(1024) unsigned char tc_raw[];
-  TcSmem& s = tc_setup(tc_raw, S);
+  TcSmem& s = tc_setup(tc_raw, P, S);
   TcEngine<MAG> eng = tc_engine<MAG>(P, S, s);
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
   for (int64_t base = ((int64_t)blockIdx.x * TC_GROUPS + eng.g) * 128; base < M;
@@ -1512,7 +1531,7 @@ static int fill_surrogate_params(const tb_field_t* field, const tb_surrogate_t* 
   memset(&S, 0, sizeof(S));
   S.wb = static_cast<const __nv_bfloat16*>(sur->weights_bf16);
   S.pf = sur->params_f32;
-  S.dom = MlpDomain{sur->r_max, sur->z_c, sur->z_half};
+  S.dom = mlp_domain(sur->r_max, sur->z_c, sur->z_half);
   S.z_lo = sur->z_lo;
   S.z_hi = sur->z_hi;
   for (int src = 0; src < nsrc; src++) {
@@ -1681,7 +1700,11 @@ static int trace_rk45(const double* start, const double* t0, const double* qm, c
   }
   cudaStream_t s = (cudaStream_t)stream;
   if (cudaMemsetAsync(work, 0, sizeof(int32_t), s) != cudaSuccess) return CUDA_ERR;
-  if (axial) return n <= (int64_t)num_sms() * 3 * 128 ? launch_axial<3>(P, s) : launch_axial<4>(P, s);
+  if (axial) {
+    const int64_t sm_round = (int64_t)num_sms() * 128;
+    const int64_t rounds3 = (n + 3 * sm_round - 1) / (3 * sm_round), rounds4 = (n + 4 * sm_round - 1) / (4 * sm_round);
+    return rounds3 == rounds4 ? launch_axial<3>(P, s) : launch_axial<4>(P, s);
+  }
   int tw = opts->team_warps;
   if (tw == 0) {
     // Fill the GPU: about 32 resident warps per SM.
