@@ -12,10 +12,11 @@
 //                  fill, tb_fill.cuh)
 //   FACT(g, i, j)  left-looking LU without pivoting, s = min(i, j):
 //                  C = A_ij - sum_{k<s} L_ik U_kj (operands staged through
-//                  shared memory by cp.async in a four-stage pipeline), then
-//                  on the diagonal the tile's own LU and the inverses of both
-//                  of its triangles, below the diagonal L_ij = C U_jj^-1,
-//                  right of it U_ij = L_ii^-1 C
+//                  shared memory by cp.async in a four-stage pipeline, each
+//                  product as soon as its two tiles are final), then on the
+//                  diagonal the inverses of both triangles of the tile's LU,
+//                  below the diagonal L_ij = C U_jj^-1, right of it
+//                  U_ij = L_ii^-1 C
 //   FWD(g, i)      y_i = L_ii^-1 (F_i - sum_{k<i} L_ik y_k)
 //   BWD(g, i)      x_i = U_ii^-1 (y_i - sum_{k>i} U_ik x_k); the block's
 //                  charges are written out and packed with their elements'
@@ -33,10 +34,20 @@
 //
 // No pivoting: these single-layer matrices factor stably without row
 // exchanges (growth factor 1 on the synthetic lenses, charges within ~1e-13
-// of LAPACK's).  A zero or non-finite pivot or charge marks the geometry
-// TB_SINGULAR, and the host solves it again with the pivoted LU.
+// of LAPACK's).  A zero or non-finite pivot or charge marks the geometry TB_SINGULAR, and
+// the host solves it again with the pivoted LU.
+//
+// What bounds it: with the late steps' few tiles the chain diagonal tile -> its
+// neighbours -> next diagonal tile.  A tile that waited for both of its last
+// factors before its first product put its whole row of products (150 us at 46
+// steps) on that chain; taken as they become final, one product is left there,
+// and the diagonal tile's 64 steps have one barrier each.  Eight mirror lenses
+// of 300 to 3,000 elements: 11.1 to 6.3 ms, of which the products take 3.6 ms
+// (half of the FP64 rate; reads of 16 bytes of both operands by 4 x 8 threads a
+// warp gave 6.29) and the fill 1.3 ms.
 #include <climits>
 #include "tb_common.cuh"
+#include "tb_fastmath.cuh"
 #include "tb_internal.cuh"
 #include "tb_fill.cuh"
 #include "../../include/traceon_b200.h"
@@ -48,9 +59,9 @@ constexpr int BTH = 256;    // threads per CTA: a 16 x 16 grid, 4 x 4 tile entri
 constexpr int KC = 16;      // inner-dimension chunk of a staged GEMM stage
 constexpr int NSTAGE = 4;   // cp.async pipeline depth
 constexpr int LDT = BT + 1; // padded row of a whole tile in shared memory
-constexpr int STAGE_DOUBLES = 2 * BT * KC;
-constexpr int SMEM_DOUBLES = 2 * BT * LDT;  // two tiles (or the GEMM stages)
-static_assert(NSTAGE * STAGE_DOUBLES <= 2 * BT * LDT, "the pipeline stages fit in the two tile buffers");
+constexpr int LDK = KC + 2; // padded row of a staged L chunk: a warp's two rows in different banks, 16-byte aligned
+constexpr int STAGE_DOUBLES = BT * LDK + KC * BT;
+constexpr int SMEM_DOUBLES = NSTAGE * STAGE_DOUBLES > 2 * BT * LDT ? NSTAGE * STAGE_DOUBLES : 2 * BT * LDT;
 static_assert(BT == FILL_TILE && BTH == FILL_THREADS && sizeof(FillTile) <= SMEM_DOUBLES * sizeof(double),
               "a FILL task is one tile of the fill");
 constexpr size_t BATCH_SMEM = SMEM_DOUBLES * sizeof(double);
@@ -104,18 +115,15 @@ __device__ __noinline__ bool thread_wait(const BatchArgs& a, const int* f, int w
       return false;
     }
     __nanosleep(ns);
-    ns = ns < 1024 ? 2 * ns : 1024;
+    ns = ns < 256 ? 2 * ns : 256;
   }
 }
 
-// The CTA waits for f0 >= w0 and, when n > 1, f1 >= w1 and f2 >= w2 (thread
-// 0 polls; the result and the acquired data reach the CTA through the
-// barrier).
-__device__ __forceinline__ bool cta_wait(const BatchArgs& a, int n, const int* f0, int w0, const int* f1 = nullptr,
-                                         int w1 = 0, const int* f2 = nullptr, int w2 = 0, int* s_ok = nullptr) {
+// The CTA waits for *f >= want (thread 0 polls; the result and the acquired
+// data reach the CTA through the barrier).
+__device__ __forceinline__ bool cta_wait(const BatchArgs& a, const int* f, int want, int* s_ok) {
   if (threadIdx.x == 0) {
-    bool ok = thread_wait(a, f0, w0);
-    if (ok && n > 1) ok = thread_wait(a, f1, w1) && thread_wait(a, f2, w2);
+    const bool ok = thread_wait(a, f, want);
     __threadfence();
     *s_ok = ok;
   }
@@ -125,8 +133,50 @@ __device__ __forceinline__ bool cta_wait(const BatchArgs& a, int n, const int* f
   return ok;
 }
 
-__device__ __forceinline__ bool cta_wait1(const BatchArgs& a, const int* f, int want, int* s_ok) {
-  return cta_wait(a, 1, f, want, nullptr, 0, nullptr, 0, s_ok);
+// How many of the tile (i, j)'s s products have both factors final, counted
+// from the first: warp 0 looks at 32 pairs of flags at a time, and waits
+// (bounded, as thread_wait) while it is no more than `done`.  The count, or 0
+// if the wait ran out.
+__device__ __forceinline__ int cta_products(const BatchArgs& a, const int* fl, int64_t T, int i, int j, int s, int done,
+                                            int* s_ok) {
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int* abort_word = a.flags + CTL_ABORT;
+    const long long t0 = clock64();
+    unsigned ns = 32;
+    int m = done;
+    for (;;) {
+      for (;;) {
+        const int k = m + lane;
+        const bool ready = k < s && b_ld_acquire(fl + (int64_t)i * T + k) >= ST_FINAL &&
+                           b_ld_acquire(fl + (int64_t)k * T + j) >= ST_FINAL;
+        const unsigned not_ready = ~__ballot_sync(0xffffffffu, ready);
+        m += not_ready ? __ffs(not_ready) - 1 : 32;
+        if (not_ready || m >= s) break;
+      }
+      if (m > done) break;
+      int stop = 0;
+      if (lane == 0) {
+        stop = *(volatile int*)abort_word != 0;
+        if (!stop && clock64() - t0 > a.wait_cycles) {
+          atomicExch(abort_word, 1);
+          stop = 1;
+        }
+      }
+      if (__shfl_sync(0xffffffffu, stop, 0)) {
+        m = 0;
+        break;
+      }
+      __nanosleep(ns);
+      ns = ns < 256 ? 2 * ns : 256;
+    }
+    __threadfence();
+    if (lane == 0) *s_ok = m;
+  }
+  __syncthreads();
+  const int m = *s_ok;
+  __syncthreads();
+  return m;
 }
 
 // Every thread's stores of the task are done (barrier), then thread 0
@@ -178,22 +228,22 @@ __device__ void task_fill(const BatchArgs& a, const tb_batch_item_t& it, int i, 
 }
 
 // ---------------------------------------------------------------- FACT
-// C (registers) -= sum_{k<s} L_ik U_kj, the operands streamed through
+// C (registers) -= sum_{k0<=k<k1} L_ik U_kj, the operands streamed through
 // NSTAGE shared-memory stages of (64 x KC) and (KC x 64).
-__device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t Np, int i, int j, int s,
+__device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t Np, int i, int j, int k0, int k1,
                                           double* sm, double (&acc)[4][4]) {
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int nq = s * (BT / KC);
+  const int nq = (k1 - k0) * (BT / KC);
   auto issue = [&](int q) {
-    const int k = q / (BT / KC), kc = q % (BT / KC);
-    double* Ls = sm + (q % NSTAGE) * STAGE_DOUBLES;  // [64][KC]
-    double* Us = Ls + BT * KC;                       // [KC][64]
+    const int k = k0 + q / (BT / KC), kc = q % (BT / KC);
+    double* Ls = sm + (q % NSTAGE) * STAGE_DOUBLES;  // [64][LDK]
+    double* Us = Ls + BT * LDK;                      // [KC][64]
     const double* Lg = A + (int64_t)i * BT * Np + (int64_t)k * BT + kc * KC;
     const double* Ug = A + ((int64_t)k * BT + kc * KC) * Np + (int64_t)j * BT;
 #pragma unroll
     for (int e = tid; e < BT * KC / 2; e += BTH) {
       const int row = e / (KC / 2), part = e % (KC / 2);
-      cp_async16(Ls + row * KC + part * 2, Lg + row * Np + part * 2);
+      cp_async16(Ls + row * LDK + part * 2, Lg + row * Np + part * 2);
     }
 #pragma unroll
     for (int e = tid; e < KC * BT / 2; e += BTH) {
@@ -211,18 +261,22 @@ __device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t 
     cp_async_wait<NSTAGE - 2>();
     __syncthreads();
     const double* Ls = sm + (q % NSTAGE) * STAGE_DOUBLES;
-    const double* Us = Ls + BT * KC;
+    const double* Us = Ls + BT * LDK;
 #pragma unroll
-    for (int kk = 0; kk < KC; kk++) {
-      double l[4], u[4];
+    for (int kk = 0; kk < KC; kk += 2) {
+      double2 l[4];
 #pragma unroll
-      for (int aa = 0; aa < 4; aa++) l[aa] = Ls[(ty + 16 * aa) * KC + kk];
+      for (int aa = 0; aa < 4; aa++) l[aa] = *reinterpret_cast<const double2*>(Ls + (ty + 16 * aa) * LDK + kk);
 #pragma unroll
-      for (int bb = 0; bb < 4; bb++) u[bb] = Us[kk * BT + tx + 16 * bb];
+      for (int h = 0; h < 2; h++) {
+        double u[4];
 #pragma unroll
-      for (int aa = 0; aa < 4; aa++)
+        for (int bb = 0; bb < 4; bb++) u[bb] = Us[(kk + h) * BT + tx + 16 * bb];
 #pragma unroll
-        for (int bb = 0; bb < 4; bb++) acc[aa][bb] = fma(-l[aa], u[bb], acc[aa][bb]);
+        for (int aa = 0; aa < 4; aa++)
+#pragma unroll
+          for (int bb = 0; bb < 4; bb++) acc[aa][bb] = fma(h ? -l[aa].y : -l[aa].x, u[bb], acc[aa][bb]);
+      }
     }
     if (q + NSTAGE - 1 < nq) issue(q + NSTAGE - 1);
     cp_async_commit();
@@ -231,66 +285,65 @@ __device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t 
   __syncthreads();
 }
 
-// LU without pivoting of the tile D (shared, [64][LDT]) in place: per step
-// the column below the pivot is scaled, then every thread updates its own
-// entries (ty + 16 aa, tx + 16 bb) of the trailing block.  Returns false on a
-// zero or non-finite pivot.
-__device__ __forceinline__ bool diag_lu(double* D) {
+// The tile's entries (ty + 16 aa, tx + 16 bb) in registers become U^-1 on and
+// above the diagonal and the strict lower part of L^-1 (whose diagonal is 1)
+// of its LU without pivoting, in one elimination in place: at step p
+//   rows r > p    l = a_rp / a_pp; the columns right of p take a_rc -= l a_pc
+//                 (the LU), those left of it, where L^-1 grows, the same, and
+//                 a_rp = -l
+//   rows r < p    z = a_rp / a_pp is U^-1's entry; right of p, where U^-1
+//                 grows, a_rc -= z a_pc
+//   row p         a_pp = 1 / a_pp, and right of p a_pc = -a_pc / a_pp
+// Row p and column p pass through shared memory in two buffers, so a step
+// costs one barrier, one reciprocal and one update of the registers.  Buffers:
+// 4 x 64 doubles.  Returns false on a zero or non-finite pivot.
+__device__ __forceinline__ bool diag_eliminate(double (&a)[4][4], double* buf) {
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   bool good = true;
+#pragma unroll
+  for (int blk = 0; blk < 4; blk++) {
+    if (tx == 0)
+#pragma unroll
+      for (int aa = 0; aa < 4; aa++) buf[ty + 16 * aa] = a[aa][blk];
+    if (ty == 0)
+#pragma unroll
+      for (int bb = 0; bb < 4; bb++) buf[2 * BT + tx + 16 * bb] = a[blk][bb];
+    __syncthreads();
 #pragma unroll 1
-  for (int p = 0; p < BT; p++) {
-    const double piv = D[p * LDT + p];
-    good = good && fabs(piv) > 0.0 && isfinite(piv);
-    if (tid > p && tid < BT) D[tid * LDT + p] /= piv;
-    __syncthreads();
+    for (int pp = 0; pp < 16; pp++) {
+      const double* col = buf + (pp & 1) * BT;
+      const double* row = buf + (2 + (pp & 1)) * BT;
+      const double piv = row[16 * blk + pp], inv = 1.0 / piv;
+      good = good && fabs(piv) > 0.0 && isfinite(piv);
+      double u[4];
 #pragma unroll
-    for (int aa = 0; aa < 4; aa++) {
-      const int r = ty + 16 * aa;
-      if (r <= p) continue;
-      const double l = D[r * LDT + p];
+      for (int bb = 0; bb < 4; bb++) u[bb] = row[tx + 16 * bb];
 #pragma unroll
-      for (int bb = 0; bb < 4; bb++) {
-        const int c = tx + 16 * bb;
-        if (c > p) D[r * LDT + c] = fma(-l, D[p * LDT + c], D[r * LDT + c]);
+      for (int aa = 0; aa < 4; aa++) {
+        const bool below = aa > blk || (aa == blk && ty > pp), pivot_row = aa == blk && ty == pp;
+        const double m = pivot_row ? inv : div_by(col[ty + 16 * aa], piv, inv);
+#pragma unroll
+        for (int bb = 0; bb < 4; bb++) {
+          const bool right = bb > blk || (bb == blk && tx > pp);
+          if (bb == blk && tx == pp)
+            a[aa][bb] = below ? -m : m;
+          else if (below || right)
+            a[aa][bb] = fma(-m, u[bb], pivot_row ? 0.0 : a[aa][bb]);
+        }
       }
+      if (pp < 15) {
+        double* next = buf + ((pp + 1) & 1) * BT;
+        if (tx == pp + 1)
+#pragma unroll
+          for (int aa = 0; aa < 4; aa++) next[ty + 16 * aa] = a[aa][blk];
+        if (ty == pp + 1)
+#pragma unroll
+          for (int bb = 0; bb < 4; bb++) next[2 * BT + tx + 16 * bb] = a[blk][bb];
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
   return good;
-}
-
-// Inverses of the two triangles of the factored tile D (shared, [64][LDT]):
-// M gets U^-1 on and above the diagonal and the strict lower part of L^-1
-// (whose diagonal is 1).  Thread pairs own one column each (pairs 0-63 of
-// U^-1, 64-127 of L^-1) and run the column's substitution, the pair's two
-// halves splitting every dot product.
-__device__ __forceinline__ void diag_inverses(const double* D, double* M) {
-  const int tid = threadIdx.x, half = tid & 1, pair = tid >> 1;
-  const bool upper = pair < BT;
-  const int c = upper ? pair : pair - BT;
-  if (upper && half == 0) M[c * LDT + c] = 1.0 / D[c * LDT + c];
-  __syncwarp();
-#pragma unroll 1
-  for (int t = 0; t < BT - 1; t++) {
-    double s = 0.0;
-    int r;
-    if (upper) {
-      r = c - 1 - t;  // X[r][c] = -sum_{q=r+1..c} U[r][q] X[q][c] / U[r][r]
-      if (r >= 0)
-        for (int q = r + 1 + half; q <= c; q += 2) s = fma(D[r * LDT + q], M[q * LDT + c], s);
-    } else {
-      r = c + 1 + t;  // X[r][c] = -sum_{q=c..r-1} L[r][q] X[q][c], X[c][c] = 1
-      if (r < BT)
-        for (int q = c + half; q < r; q += 2) s = fma(D[r * LDT + q], q == c ? 1.0 : M[q * LDT + c], s);
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    if (half == 0) {
-      if (upper && r >= 0) M[r * LDT + c] = -s / D[r * LDT + r];
-      if (!upper && r < BT) M[r * LDT + c] = -s;
-    }
-    __syncwarp();
-  }
 }
 
 __device__ bool task_fact(const BatchArgs& a, const tb_batch_item_t& it, int g, int i, int j, double* sm, int* s_ok) {
@@ -299,35 +352,33 @@ __device__ bool task_fact(const BatchArgs& a, const tb_batch_item_t& it, int g, 
   double* A = a.work + it.a_off;
   int* fl = tile_flags(a, it);
   const int s = i < j ? i : j;
-  // this tile filled; the tiles of step s - 1 in its row and column final
-  if (!cta_wait(a, s > 0 ? 3 : 1, fl + (int64_t)i * T + j, ST_FILLED, fl + (int64_t)i * T + (s - 1), ST_FINAL,
-                fl + (int64_t)(s - 1) * T + j, ST_FINAL, s_ok))
-    return false;
+  if (!cta_wait(a, fl + (int64_t)i * T + j, ST_FILLED, s_ok)) return false;
   double acc[4][4];
 #pragma unroll
   for (int aa = 0; aa < 4; aa++)
 #pragma unroll
     for (int bb = 0; bb < 4; bb++)
       acc[aa][bb] = __ldcg(A + ((int64_t)i * BT + ty + 16 * aa) * Np + (int64_t)j * BT + tx + 16 * bb);
-  fact_gemm(A, Np, i, j, s, sm, acc);
+  for (int done = 0; done < s;) {
+    const int m = cta_products(a, fl, T, i, j, s, done, s_ok);
+    if (m <= done) return false;
+    fact_gemm(A, Np, i, j, done, m, sm, acc);
+    done = m;
+  }
   double* D = sm;
   double* M = sm + BT * LDT;
   if (i == j) {
+    const bool good = diag_eliminate(acc, sm);
+    if (tid == 0 && !good) atomicOr(fl + T * T + 2 * T, 1);
+    double* inv = a.work + it.inv_off + (int64_t)i * BT * BT;
 #pragma unroll
     for (int aa = 0; aa < 4; aa++)
 #pragma unroll
-      for (int bb = 0; bb < 4; bb++) D[(ty + 16 * aa) * LDT + tx + 16 * bb] = acc[aa][bb];
-    __syncthreads();
-    const bool good = diag_lu(D);
-    if (tid == 0 && !good) atomicOr(fl + T * T + 2 * T, 1);
-    diag_inverses(D, M);
-    __syncthreads();
-    double* inv = a.work + it.inv_off + (int64_t)i * BT * BT;
-    for (int e = tid; e < BT * BT; e += BTH) inv[e] = M[(e >> 6) * LDT + (e & 63)];
+      for (int bb = 0; bb < 4; bb++) inv[(ty + 16 * aa) * BT + tx + 16 * bb] = acc[aa][bb];
     publish(fl + (int64_t)i * T + j, ST_FINAL);
     return true;
   }
-  if (!cta_wait1(a, fl + (int64_t)s * T + s, ST_FINAL, s_ok)) return false;
+  if (!cta_wait(a, fl + (int64_t)s * T + s, ST_FINAL, s_ok)) return false;
   const bool lower = i > j;
   const double* inv = a.work + it.inv_off + (int64_t)s * BT * BT;
 #pragma unroll
@@ -396,7 +447,7 @@ __device__ bool task_fwd(const BatchArgs& a, const tb_batch_item_t& it, int i, d
   int* fl = tile_flags(a, it);
   int* yd = fl + T * T;
   // the diagonal tile final implies every tile left of it and above it
-  if (!cta_wait1(a, fl + (int64_t)i * T + i, ST_FINAL, s_ok)) return false;
+  if (!cta_wait(a, fl + (int64_t)i * T + i, ST_FINAL, s_ok)) return false;
   const double* Lrow = A + ((int64_t)i * BT + rr) * Np + part * 16;
   double acc = 0.0;
 #pragma unroll 1
@@ -408,7 +459,7 @@ __device__ bool task_fwd(const BatchArgs& a, const tb_batch_item_t& it, int i, d
       l[q] = mm.x;
       l[q + 1] = mm.y;
     }
-    if (!cta_wait1(a, yd + k, 1, s_ok)) return false;
+    if (!cta_wait(a, yd + k, 1, s_ok)) return false;
     const double* yk = v + (int64_t)k * BT + part * 16;
 #pragma unroll
     for (int q = 0; q < 16; q++) acc = fma(l[q], __ldcg(yk + q), acc);
@@ -442,7 +493,7 @@ __device__ bool task_bwd(const BatchArgs& a, const tb_batch_item_t& it, int g, i
   int* yd = fl + T * T;
   int* xd = yd + T;
   // the last forward block implies every factor tile and every y block
-  if (!cta_wait1(a, yd + (T - 1), 1, s_ok)) return false;
+  if (!cta_wait(a, yd + (T - 1), 1, s_ok)) return false;
   const double* Urow = A + ((int64_t)i * BT + rr) * Np + part * 16;
   double acc = 0.0;
 #pragma unroll 1
@@ -454,7 +505,7 @@ __device__ bool task_bwd(const BatchArgs& a, const tb_batch_item_t& it, int g, i
       l[q] = mm.x;
       l[q + 1] = mm.y;
     }
-    if (!cta_wait1(a, xd + k, 1, s_ok)) return false;
+    if (!cta_wait(a, xd + k, 1, s_ok)) return false;
     const double* xk = v + k * BT + part * 16;
 #pragma unroll
     for (int q = 0; q < 16; q++) acc = fma(l[q], __ldcg(xk + q), acc);
