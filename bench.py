@@ -396,7 +396,7 @@ def precision_solve(n, nrhs=8, seed=2, field_points=1 << 20, fp64_lu=True, fp64_
     # terms are computed and overwritten, as in the reference)
     pots = float(n) * n * 16
     out['fill_roofline'] = fp64_roofline(pots, FLOP_RING_POT, fill_ms, fp64_peak, 'k_fill_matrix',
-                                         'ring-potential evaluations (+ 1 log, 1 rsqrt each)')
+                                         'ring-potential evaluations of the 16-point rule', direct=False)
     del A
     torch.cuda.empty_cache()
     if field_points:
@@ -409,11 +409,13 @@ def precision_solve(n, nrhs=8, seed=2, field_points=1 << 20, fp64_lu=True, fp64_
     return out
 
 
-def fp64_roofline(units, flop_per_unit, ms, peak, kernel, unit_desc):
+def fp64_roofline(units, flop_per_unit, ms, peak, kernel, unit_desc, direct=True):
+    """direct=False: the kernel does not compute each unit (ring tree, short Gauss rules), so the rate of the units
+    that it stands for is no fraction of the peak."""
     achieved = units * flop_per_unit / (ms * 1e-3) / 1e12
     return {'bound': 'fp64', 'kernel': kernel, 'units': units, 'flop_per_unit': flop_per_unit,
             'unit_desc': unit_desc, 'achieved': achieved, 'unit': 'TFLOP/s', 'peak': peak,
-            'frac': achieved / peak if peak else None,
+            'frac': achieved / peak if peak and direct else None, 'counts': 'computed' if direct else 'direct-sum units',
             'peak_source': 'FP64 FMA throughput measured in this run (tests/probe tb_probe_fp64_fma)'}
 
 
@@ -442,8 +444,7 @@ def precision_fields(geo, charges_t, m, seed, fp64_peak=None):
     pairs = float(m) * src.shape[1]
     return {'field_points': m, 'field_ms': ms, 'field_ring_pairs_per_s': pairs / (ms * 1e-3),
             'field_roofline': fp64_roofline(pairs, FLOP_FIELD_PAIR_POT, ms, fp64_peak, 'k_field_points',
-                                            'ring-pair potential + field evaluations (+ 1 log, 1 rsqrt, '
-                                            '1 reciprocal each)'),
+                                            'ring-pair potential + field evaluations of the direct sums', direct=False),
             '_field_state': (geo.vertices, charges_t.cpu().numpy(), pts, pot.cpu().numpy(), fld.cpu().numpy(), seed)}
 
 
@@ -759,8 +760,9 @@ def run_gpu(args):
                                 'kernel': 'k_trace_bem',
                                 'roofline': {'bound': 'fp64', 'unit': 'TFLOP/s', 'flop_per_pair': FLOP_FIELD_PAIR,
                                              'achieved': pairs * FLOP_FIELD_PAIR / launch_s / 1e12,
-                                             'unit_desc': 'ring-pair field evaluations, algorithmic FP64 flops '
-                                                          '(+ 1 log, 1 rsqrt, 1 reciprocal per pair)'}}
+                                             'counts': 'direct-sum units', 'frac': None,
+                                             'unit_desc': 'ring-pair field evaluations of the direct sums, which the '
+                                                          'tracer takes through its ring tree'}}
             row['speedup_surrogate_vs_plain_bem'] = row['surrogate']['value'] / row['plain_bem']['value']
             row['speedup_axial_only_vs_plain_bem'] = row['axial_only']['value'] / row['plain_bem']['value']
             # errors against the GPU FP64 BEM trace of the slice (itself
@@ -800,16 +802,15 @@ def run_gpu(args):
         for row in arms.values():
             rf = row['plain_bem']['roofline']
             rf['peak'] = fp64_peak
-            rf['frac'] = rf['achieved'] / fp64_peak
             rf['peak_source'] = 'FP64 FMA throughput measured in this run (tests/probe tb_probe_fp64_fma)'
     else:
         pairs_per_launch = attempts * 6 * Nq
         achieved = pairs_per_launch * FLOP_FIELD_PAIR / launch_s / 1e12
         roof = {'bound': 'fp64', 'achieved': achieved, 'peak': fp64_peak, 'unit': 'TFLOP/s',
-                'frac': achieved / fp64_peak if fp64_peak else None, 'traffic': None, 'kernel': 'k_trace_bem',
+                'frac': None, 'counts': 'direct-sum units', 'traffic': None, 'kernel': 'k_trace_bem',
                 'flop_per_unit': FLOP_FIELD_PAIR, 'units_per_launch': pairs_per_launch,
-                'unit_desc': 'ring-pair field evaluations, algorithmic FP64 flops (+ 1 log, 1 rsqrt, '
-                             '1 reciprocal per pair)',
+                'unit_desc': 'ring-pair field evaluations of the direct sums, which the tracer takes through its ring '
+                             'tree',
                 'peak_source': 'FP64 FMA throughput measured in this run (tests/probe tb_probe_fp64_fma)'}
 
     precision = precision_solve(args.precision_n, fp64_peak=fp64_peak, field_points=args.field_points,

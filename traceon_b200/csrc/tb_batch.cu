@@ -6,7 +6,7 @@
 // Every geometry's matrix is padded to T x T tiles of 64 x 64 (identity on
 // the padded diagonal, zeros elsewhere) in a workspace that
 // tb_batch_solve_plan lays out; the plan also lists the tile tasks:
-//   FILL(g, i, j)  the tile's entries: the 16-point Gauss sums of
+//   FILL(g, i, j)  the tile's entries: the Gauss sums of
 //                  radial.c:249-310 off the diagonal and the singular self
 //                  terms on it (the device functions of the one-geometry
 //                  fill, tb_fill.cuh)
@@ -34,8 +34,8 @@
 //
 // No pivoting: these single-layer matrices factor stably without row
 // exchanges (growth factor 1 on the synthetic lenses, charges within ~1e-13
-// of LAPACK's).  A zero or non-finite pivot or charge marks the geometry TB_SINGULAR, and
-// the host solves it again with the pivoted LU.
+// of LAPACK's).  A zero or non-finite pivot or charge marks the geometry
+// TB_SINGULAR, and the host solves it again with the pivoted LU.
 //
 // What bounds it: with the late steps' few tiles the chain diagonal tile -> its
 // neighbours -> next diagonal tile.  A tile that waited for both of its last

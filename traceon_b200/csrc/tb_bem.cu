@@ -1,15 +1,16 @@
 // tb_bem.cu -- BEM assembly and field-sum kernels of the radial path.
 //
 //   jacobian buffer      radial.c:224-246
-//   matrix fill          radial.c:249-310 (off-diagonal 16-point Gauss sums)
+//   matrix fill          radial.c:249-310 (off-diagonal Gauss sums, tb_fill.cuh)
 //   self integrals       radial.c:182-222 + traceon/backend/__init__.py:688-708
 //   potential / field    radial.c:105-173, batched over points
 //   axial derivatives    radial.c:18-36
 //   axial coefficients   traceon/field.py:914-937
 //   axial evaluation     radial.c:312-384, batched over points
 //
-// Everything is FP64; the kernels are FP64-pipe bound (one log, one sqrt and
-// one division per ring pair).
+// Everything is FP64.  The sums over rings are FP64-pipe bound (one reciprocal
+// square root and a table logarithm per ring pair); large maps go through the
+// ring tree (tb_tree.cu), a few points take a cluster of CTAs each.
 #include <cooperative_groups.h>
 
 #include "tb_common.cuh"

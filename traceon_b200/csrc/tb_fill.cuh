@@ -1,5 +1,5 @@
 // tb_fill.cuh -- matrix entries of the radial BEM fill: the off-diagonal
-// 16-point Gauss sums and the singular self terms, shared by the single-
+// Gauss sums and the singular self terms, shared by the single-
 // geometry kernels and the batched persistent solve.
 #pragma once
 

@@ -4,7 +4,8 @@
 // Particles are pulled from a device work queue by teams.  For BEM fields a
 // team is 1-8 warps that split the ring sums of every field evaluation
 // (field_radial_traceable, tracing.c:125-165) and reduce them with shuffles
-// (and a named barrier across warps); every lane of a team then holds the
+// (and a named barrier across warps), through the ring tree of tb_tree.cuh for
+// electrostatic fields where the caller gives a workspace; every lane of a team then holds the
 // same field bits, so the step control runs redundantly and uniformly in all
 // lanes.  For axial-interpolated fields (field_radial_derivs_traceable,
 // tracing.c:168-174) a team is one thread.
