@@ -41,10 +41,11 @@
 // neighbours -> next diagonal tile.  A tile that waited for both of its last
 // factors before its first product put its whole row of products (150 us at 46
 // steps) on that chain; taken as they become final, one product is left there,
-// and the diagonal tile's 64 steps have one barrier each.  Eight mirror lenses
-// of 300 to 3,000 elements: 11.1 to 6.3 ms, of which the products take 3.6 ms
-// (half of the FP64 rate; reads of 16 bytes of both operands by 4 x 8 threads a
-// warp gave 6.29) and the fill 1.3 ms.
+// and the diagonal tile's 64 steps have one barrier each (eight mirror lenses
+// of 300 to 3,000 elements: 11.1 to 6.3 ms).  Beside the chain the products:
+// with 4 x 4 entries a thread each 16 FMAs wait for 8 doubles from shared
+// memory, whose 128 bytes a cycle then hold the FP64 pipe at half its rate;
+// matrix instructions read an eighth of that (6.3 to 5.3 ms).
 #include <climits>
 #include "tb_common.cuh"
 #include "tb_fastmath.cuh"
@@ -55,13 +56,16 @@
 namespace tb {
 
 constexpr int BT = 64;      // tile edge
-constexpr int BTH = 256;    // threads per CTA: a 16 x 16 grid, 4 x 4 tile entries each
+constexpr int BTH = 256;    // threads per CTA: 8 warps, 16 x 32 tile entries each in the products
 constexpr int KC = 16;      // inner-dimension chunk of a staged GEMM stage
 constexpr int NSTAGE = 4;   // cp.async pipeline depth
-constexpr int LDT = BT + 1; // padded row of a whole tile in shared memory
-constexpr int LDK = KC + 2; // padded row of a staged L chunk: a warp's two rows in different banks, 16-byte aligned
-constexpr int STAGE_DOUBLES = BT * LDK + KC * BT;
-constexpr int SMEM_DOUBLES = NSTAGE * STAGE_DOUBLES > 2 * BT * LDT ? NSTAGE * STAGE_DOUBLES : 2 * BT * LDT;
+// Rows in shared memory are padded to 4 mod 16 doubles: the fragments of
+// dmma, 8 rows by 4 entries, then lie in different banks.
+constexpr int LDT = BT + 4;  // row of a whole tile, and of a staged U chunk
+constexpr int LDK = KC + 4;  // row of a staged L chunk
+constexpr int STAGE_DOUBLES = BT * LDK + KC * LDT;
+constexpr int SMEM_DOUBLES = NSTAGE * STAGE_DOUBLES;
+static_assert(SMEM_DOUBLES >= 2 * BT * LDT, "the two tile buffers fit in the pipeline stages");
 static_assert(BT == FILL_TILE && BTH == FILL_THREADS && sizeof(FillTile) <= SMEM_DOUBLES * sizeof(double),
               "a FILL task is one tile of the fill");
 constexpr size_t BATCH_SMEM = SMEM_DOUBLES * sizeof(double);
@@ -228,16 +232,78 @@ __device__ void task_fill(const BatchArgs& a, const tb_batch_item_t& it, int i, 
 }
 
 // ---------------------------------------------------------------- FACT
+// A warp's part of a tile's product is 16 rows by 32 columns, by FP64 matrix
+// instructions (m16n8k8).  Lane l holds rows row and row + 8 (row = 16 (warp /
+// 2) + l / 4) and columns col + 8 n and the next (col = 32 (warp % 2) + 2 (l %
+// 4)): c[n] = {(row, col + 8 n), +1, (row + 8, col + 8 n), +1}.
+struct TileLane {
+  int row, col, k, n;  // k, n: the lane's entry of an operand fragment, l % 4 and l / 4
+  __device__ __forceinline__ TileLane() {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    k = lane & 3;
+    n = lane >> 2;
+    row = 16 * (warp >> 1) + n;
+    col = 32 * (warp & 1) + 2 * k;
+  }
+};
+
+// c += a b, a 16 x 8 (entries (n, k), (n + 8, k), (n, k + 4), (n + 8, k + 4)
+// in a lane), b 8 x 8 (entries (k, n), (k + 4, n)).
+__device__ __forceinline__ void dmma(double (&c)[4], const double (&a)[4], double b0, double b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+
+// c += (or -=) X Y over K entries, X's rows of ldx and Y's of LDT in shared
+// memory.
+template <int K, bool MINUS>
+__device__ __forceinline__ void tile_product(const TileLane& t, const double* X, int ldx, const double* Y,
+                                             double (&c)[4][4]) {
+  const double* x = X + t.row * ldx + t.k;
+  const double* y = Y + t.k * LDT + (t.col - 2 * t.k) + t.n;
+#pragma unroll 2
+  for (int q = 0; q < K; q += 8) {
+    double a[4] = {x[q], x[8 * ldx + q], x[q + 4], x[8 * ldx + q + 4]};
+    if (MINUS) {
+#pragma unroll
+      for (int e = 0; e < 4; e++) a[e] = -a[e];
+    }
+#pragma unroll
+    for (int n = 0; n < 4; n++) dmma(c[n], a, y[q * LDT + 8 * n], y[(q + 4) * LDT + 8 * n]);
+  }
+}
+
+// A tile's entries in that layout, from and to rows of ld.
+__device__ __forceinline__ void tile_load(const double* src, int64_t ld, const TileLane& t, double (&c)[4][4]) {
+#pragma unroll
+  for (int n = 0; n < 4; n++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const double2 v = __ldcg(reinterpret_cast<const double2*>(src + (t.row + 8 * h) * ld + t.col + 8 * n));
+      c[n][2 * h] = v.x;
+      c[n][2 * h + 1] = v.y;
+    }
+}
+__device__ __forceinline__ void tile_store(double* dst, int64_t ld, const TileLane& t, const double (&c)[4][4]) {
+#pragma unroll
+  for (int n = 0; n < 4; n++)
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      *reinterpret_cast<double2*>(dst + (t.row + 8 * h) * ld + t.col + 8 * n) = double2{c[n][2 * h], c[n][2 * h + 1]};
+}
+
 // C (registers) -= sum_{k0<=k<k1} L_ik U_kj, the operands streamed through
 // NSTAGE shared-memory stages of (64 x KC) and (KC x 64).
 __device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t Np, int i, int j, int k0, int k1,
-                                          double* sm, double (&acc)[4][4]) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+                                          double* sm, const TileLane& t, double (&acc)[4][4]) {
+  const int tid = threadIdx.x;
   const int nq = (k1 - k0) * (BT / KC);
   auto issue = [&](int q) {
     const int k = k0 + q / (BT / KC), kc = q % (BT / KC);
     double* Ls = sm + (q % NSTAGE) * STAGE_DOUBLES;  // [64][LDK]
-    double* Us = Ls + BT * LDK;                      // [KC][64]
+    double* Us = Ls + BT * LDK;                      // [KC][LDT]
     const double* Lg = A + (int64_t)i * BT * Np + (int64_t)k * BT + kc * KC;
     const double* Ug = A + ((int64_t)k * BT + kc * KC) * Np + (int64_t)j * BT;
 #pragma unroll
@@ -248,7 +314,7 @@ __device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t 
 #pragma unroll
     for (int e = tid; e < KC * BT / 2; e += BTH) {
       const int row = e / (BT / 2), part = e % (BT / 2);
-      cp_async16(Us + row * BT + part * 2, Ug + row * Np + part * 2);
+      cp_async16(Us + row * LDT + part * 2, Ug + row * Np + part * 2);
     }
   };
 #pragma unroll
@@ -261,23 +327,7 @@ __device__ __forceinline__ void fact_gemm(const double* __restrict__ A, int64_t 
     cp_async_wait<NSTAGE - 2>();
     __syncthreads();
     const double* Ls = sm + (q % NSTAGE) * STAGE_DOUBLES;
-    const double* Us = Ls + BT * LDK;
-#pragma unroll
-    for (int kk = 0; kk < KC; kk += 2) {
-      double2 l[4];
-#pragma unroll
-      for (int aa = 0; aa < 4; aa++) l[aa] = *reinterpret_cast<const double2*>(Ls + (ty + 16 * aa) * LDK + kk);
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        double u[4];
-#pragma unroll
-        for (int bb = 0; bb < 4; bb++) u[bb] = Us[(kk + h) * BT + tx + 16 * bb];
-#pragma unroll
-        for (int aa = 0; aa < 4; aa++)
-#pragma unroll
-          for (int bb = 0; bb < 4; bb++) acc[aa][bb] = fma(h ? -l[aa].y : -l[aa].x, u[bb], acc[aa][bb]);
-      }
-    }
+    tile_product<KC, true>(t, Ls, LDK, Ls + BT * LDK, acc);
     if (q + NSTAGE - 1 < nq) issue(q + NSTAGE - 1);
     cp_async_commit();
   }
@@ -347,44 +397,46 @@ __device__ __forceinline__ bool diag_eliminate(double (&a)[4][4], double* buf) {
 }
 
 __device__ bool task_fact(const BatchArgs& a, const tb_batch_item_t& it, int g, int i, int j, double* sm, int* s_ok) {
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int tid = threadIdx.x;
+  const TileLane t;
   const int64_t T = it.T, Np = T * BT;
   double* A = a.work + it.a_off;
+  double* tile = A + (int64_t)i * BT * Np + (int64_t)j * BT;
   int* fl = tile_flags(a, it);
   const int s = i < j ? i : j;
   if (!cta_wait(a, fl + (int64_t)i * T + j, ST_FILLED, s_ok)) return false;
   double acc[4][4];
-#pragma unroll
-  for (int aa = 0; aa < 4; aa++)
-#pragma unroll
-    for (int bb = 0; bb < 4; bb++)
-      acc[aa][bb] = __ldcg(A + ((int64_t)i * BT + ty + 16 * aa) * Np + (int64_t)j * BT + tx + 16 * bb);
+  tile_load(tile, Np, t, acc);
   for (int done = 0; done < s;) {
     const int m = cta_products(a, fl, T, i, j, s, done, s_ok);
     if (m <= done) return false;
-    fact_gemm(A, Np, i, j, done, m, sm, acc);
+    fact_gemm(A, Np, i, j, done, m, sm, t, acc);
     done = m;
   }
   double* D = sm;
   double* M = sm + BT * LDT;
+  tile_store(D, LDT, t, acc);
   if (i == j) {
-    const bool good = diag_eliminate(acc, sm);
+    const int tx = tid & 15, ty = tid >> 4;  // the elimination's layout
+    double d[4][4];
+    __syncthreads();
+#pragma unroll
+    for (int aa = 0; aa < 4; aa++)
+#pragma unroll
+      for (int bb = 0; bb < 4; bb++) d[aa][bb] = D[(ty + 16 * aa) * LDT + tx + 16 * bb];
+    const bool good = diag_eliminate(d, M);
     if (tid == 0 && !good) atomicOr(fl + T * T + 2 * T, 1);
     double* inv = a.work + it.inv_off + (int64_t)i * BT * BT;
 #pragma unroll
     for (int aa = 0; aa < 4; aa++)
 #pragma unroll
-      for (int bb = 0; bb < 4; bb++) inv[(ty + 16 * aa) * BT + tx + 16 * bb] = acc[aa][bb];
+      for (int bb = 0; bb < 4; bb++) inv[(ty + 16 * aa) * BT + tx + 16 * bb] = d[aa][bb];
     publish(fl + (int64_t)i * T + j, ST_FINAL);
     return true;
   }
   if (!cta_wait(a, fl + (int64_t)s * T + s, ST_FINAL, s_ok)) return false;
   const bool lower = i > j;
   const double* inv = a.work + it.inv_off + (int64_t)s * BT * BT;
-#pragma unroll
-  for (int aa = 0; aa < 4; aa++)
-#pragma unroll
-    for (int bb = 0; bb < 4; bb++) D[(ty + 16 * aa) * LDT + tx + 16 * bb] = acc[aa][bb];
   // below the diagonal U_ss^-1 (zeros under it), right of it L_ss^-1 (ones on
   // the diagonal, zeros above it)
   for (int e = tid; e < BT * BT; e += BTH) {
@@ -393,26 +445,12 @@ __device__ bool task_fact(const BatchArgs& a, const tb_batch_item_t& it, int g, 
     M[r * LDT + c] = lower ? (r <= c ? v : 0.0) : (r > c ? v : (r == c ? 1.0 : 0.0));
   }
   __syncthreads();
-  const double* X = lower ? D : M;  // out = X Y
-  const double* Y = lower ? M : D;
   double out[4][4] = {};
-#pragma unroll 4
-  for (int q = 0; q < BT; q++) {
-    double x[4], y[4];
-#pragma unroll
-    for (int aa = 0; aa < 4; aa++) x[aa] = X[(ty + 16 * aa) * LDT + q];
-#pragma unroll
-    for (int bb = 0; bb < 4; bb++) y[bb] = Y[q * LDT + tx + 16 * bb];
-#pragma unroll
-    for (int aa = 0; aa < 4; aa++)
-#pragma unroll
-      for (int bb = 0; bb < 4; bb++) out[aa][bb] = fma(x[aa], y[bb], out[aa][bb]);
-  }
-#pragma unroll
-  for (int aa = 0; aa < 4; aa++)
-#pragma unroll
-    for (int bb = 0; bb < 4; bb++)
-      A[((int64_t)i * BT + ty + 16 * aa) * Np + (int64_t)j * BT + tx + 16 * bb] = out[aa][bb];
+  if (lower)
+    tile_product<BT, false>(t, D, LDT, M, out);
+  else
+    tile_product<BT, false>(t, M, LDT, D, out);
+  tile_store(tile, Np, t, out);
   publish(fl + (int64_t)i * T + j, ST_FINAL);
   return true;
 }
