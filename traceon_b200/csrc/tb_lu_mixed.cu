@@ -1249,28 +1249,81 @@ static int lookahead_reserve() {
   return v < 0 ? num_sms() / 5 : v;
 }
 
+// The side streams.  Enqueueing a factorisation records and awaits the three
+// events in turn, so it has a stream and events to itself until it returns
+// (host threads may solve at the same time): SideLease takes one of the
+// device's SIDE_SLOTS and gives it back.  What the calls have queued by then no
+// longer depends on the events, and a later call's work on the side stream
+// comes after it.  A side stream that is part of a capture that has not ended
+// serves that capture only.  With every slot taken the factorisation runs
+// without lookahead, which gives the same factors bit for bit.
+constexpr int SIDE_SLOTS = 8;
 struct SideStream {
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, top = nullptr, bottom = nullptr;
+  bool taken = false;
 };
 static std::mutex g_side_mutex;
-static SideStream g_side[64];
+static SideStream g_side[64][SIDE_SLOTS];
 
-static int side_stream(SideStream*& out) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return CUDA_ERR;
-  std::lock_guard<std::mutex> lock(g_side_mutex);
-  SideStream& ss = g_side[dev];
-  if (!ss.side) {
-    if (cudaStreamCreateWithFlags(&ss.side, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ss.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ss.top, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&ss.bottom, cudaEventDisableTiming) != cudaSuccess)
-      return CUDA_ERR;
-  }
-  out = &ss;
-  return OK;
+// The capture that s is part of, 0 for none.
+static unsigned long long capture_of(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) return 0;
+  if (status == cudaStreamCaptureStatusInvalidated) return ~0ull;
+  return status == cudaStreamCaptureStatusActive ? id : 0;
 }
+
+class SideLease {
+ public:
+  SideLease() = default;
+  SideLease(const SideLease&) = delete;
+  SideLease& operator=(const SideLease&) = delete;
+  ~SideLease() {
+    if (!ss_) return;
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    ss_->taken = false;
+  }
+  // The slot, for a call on s, or null when none is free (then OK too).
+  int take(cudaStream_t s, SideStream*& out) {
+    int dev = 0;
+    out = nullptr;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return CUDA_ERR;
+    const unsigned long long here = capture_of(s);
+    std::lock_guard<std::mutex> lock(g_side_mutex);
+    for (SideStream& ss : g_side[dev]) {
+      if (ss.taken) continue;
+      if (ss.side) {
+        const unsigned long long there = capture_of(ss.side);
+        if (there != 0 && there != here) continue;
+      } else if (make(ss) != OK) {
+        return CUDA_ERR;
+      }
+      ss.taken = true;
+      ss_ = out = &ss;
+      return OK;
+    }
+    return OK;
+  }
+
+ private:
+  static int make(SideStream& ss) {
+    SideStream x;
+    if (cudaStreamCreateWithFlags(&x.side, cudaStreamNonBlocking) == cudaSuccess &&
+        cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&x.top, cudaEventDisableTiming) == cudaSuccess &&
+        cudaEventCreateWithFlags(&x.bottom, cudaEventDisableTiming) == cudaSuccess) {
+      ss = x;
+      return OK;
+    }
+    for (cudaEvent_t e : {x.fork, x.top, x.bottom})
+      if (e) cudaEventDestroy(e);
+    if (x.side) cudaStreamDestroy(x.side);
+    return CUDA_ERR;
+  }
+  SideStream* ss_ = nullptr;
+};
 
 static int64_t lu_tc_bytes(int64_t N) {
   // two alternating split-operand buffers and the panel's scratch area
@@ -1301,8 +1354,9 @@ static int panel_attr() {
 // wait ran out.
 static int lu_nopiv_f32_tc(float* A, int64_t lda, int64_t N, int* err, uint8_t* work, cudaStream_t s) {
   const int reserve = lookahead_reserve();
+  SideLease lease;
   SideStream* ss = nullptr;
-  if (reserve > 0 && side_stream(ss) != OK) return CUDA_ERR;
+  if (reserve > 0 && lease.take(s, ss) != OK) return CUDA_ERR;
   if (gemm_pre_attr() != OK || panel_attr() != OK) return CUDA_ERR;
   PanelScratch* scratch =
       reinterpret_cast<PanelScratch*>(work + 2 * round256(gemm_pre_bytes(N, N, TC_PANEL)));
