@@ -106,9 +106,11 @@ int tree_build(const Tree& T, const double* src, const int64_t* offsets, cudaStr
 
 // Scratch of one warp's walk.  A round of the walk takes at most 32 nodes off
 // the stack and puts at most 64 children on it, the deepest first, so each
-// level of the tree (at most 18) leaves at most 32 nodes behind.
+// level of the tree (at most 18) leaves at most 32 nodes behind.  It puts at
+// most 32 TREE_LEAF chunks on the list, which is emptied above TREE_FLUSH.
 constexpr int TREE_STACK = 32 * 18 + 64;
-constexpr int TREE_LIST = 96;
+constexpr int TREE_FLUSH = 64;
+constexpr int TREE_LIST = TREE_FLUSH + 32 * TREE_LEAF;
 struct TreeScratch {
   int stack[TREE_STACK];
   int list[TREE_LIST];
@@ -116,22 +118,35 @@ struct TreeScratch {
 
 // Adds this lane's share of the field sums of groups' runs run0 .. run1 - 1 at
 // (r0, z0) to Sr, Sz (Sp); all lanes of the warp call it.  `part` of `parts`
-// warps take the chunks in turn (each walks the tree for itself).
+// (a power of two) warps take the chunks in turn (each walks the tree for
+// itself).
+//
+// Proxies and the elements of leaves that are too near for theirs go to one
+// list of chunks, a half-warp per chunk, and each list starts with the
+// half-warp after the one that took the last chunk of the one before: however
+// short the runs are, all half-warps of all parts have the same number of
+// rings to within one chunk (a half-warp per leaf, one leaf after another,
+// left all but one idle on meshes whose neighbours are not on one line: 800
+// elements in random order, one electron and eight warps 38 ms instead of the
+// direct sums' 3.1).
 template <bool POT>
 __device__ __forceinline__ void tree_sums(const Tree& T, int run0, int run1, double r0, double z0, TreeScratch& sc,
                                           int part, int parts, double& Sr, double& Sz, double& Sp) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   const double* mine = T.chunk + (lane & 15);
-  const int half = (lane >> 4) + 2 * part, step = 2 * parts;
+  const int step = 2 * parts;
+  int turn = (lane >> 4) + 2 * part;  // this half-warp's first chunk of the next list
   int nst = 0, nl = 0;
+  auto add = [&](int chunk) {
+    const double* p = mine + int64_t(chunk) * TREE_CHUNK;
+    ring_field_acc<POT>(r0, z0, p[0], p[TREE_P], p[2 * TREE_P], Sr, Sz, Sp);
+  };
   auto flush = [&]() {
     __syncwarp();
 #pragma unroll 2
-    for (int i = half; i < nl; i += step) {
-      const double* p = mine + int64_t(sc.list[i]) * TREE_CHUNK;
-      ring_field_acc<POT>(r0, z0, p[0], p[TREE_P], p[2 * TREE_P], Sr, Sz, Sp);
-    }
+    for (int i = turn; i < nl; i += step) add(sc.list[i]);
+    turn = (turn - nl) & (step - 1);
     __syncwarp();
     nl = 0;
   };
@@ -158,8 +173,9 @@ __device__ __forceinline__ void tree_sums(const Tree& T, int run0, int run1, dou
       use = ne > 0 && sqrtf(fmaf(a, a, v2)) + sqrtf(fmaf(b, b, v2)) >= nd.reach;
       split = ne > 0 && !use && !(nd.tag & 4);
     }
+    const bool near = ne > 0 && !use && !split;  // too near for the leaf's proxies: its elements' rings
     const unsigned mu = __ballot_sync(0xffffffffu, use), ms = __ballot_sync(0xffffffffu, split);
-    unsigned ml = __ballot_sync(0xffffffffu, ne > 0 && !use && !split);
+    const unsigned mn = __ballot_sync(0xffffffffu, near);
     if (use) sc.list[nl + __popc(mu & below)] = T.n + slot;
     nl += __popc(mu);
     if (split) {
@@ -168,17 +184,25 @@ __device__ __forceinline__ void tree_sums(const Tree& T, int run0, int run1, dou
       sc.stack[at + 1] = link + 1;
     }
     nst += 2 * __popc(ms);
-    while (ml) {  // too near for the leaf's proxies: its rings, element by element
-      const int src = __ffs(ml) - 1;
-      ml &= ml - 1;
-      const int le0 = __shfl_sync(0xffffffffu, link, src), lne = __shfl_sync(0xffffffffu, ne, src);
+    if (mn) {
+      // up to four chunks a leaf, at the sum of the lower lanes' counts
+      const int c = near && ne <= TREE_LEAF ? ne : 0;
+      const unsigned c1 = __ballot_sync(0xffffffffu, c & 1), c2 = __ballot_sync(0xffffffffu, c & 2),
+                     c4 = __ballot_sync(0xffffffffu, c & 4);
+      const int at = nl + __popc(c1 & below) + 2 * __popc(c2 & below) + 4 * __popc(c4 & below);
+      for (int k = 0; k < c; k++) sc.list[at + k] = link + k;
+      nl += __popc(c1) + 2 * __popc(c2) + 4 * __popc(c4);
+      unsigned ml = __ballot_sync(0xffffffffu, near && ne > TREE_LEAF);
+      while (ml) {  // a long run without proxies
+        const int src = __ffs(ml) - 1;
+        ml &= ml - 1;
+        const int le0 = __shfl_sync(0xffffffffu, link, src), lne = __shfl_sync(0xffffffffu, ne, src);
 #pragma unroll 2
-      for (int i = half; i < lne; i += step) {
-        const double* p = mine + int64_t(le0 + i) * TREE_CHUNK;
-        ring_field_acc<POT>(r0, z0, p[0], p[TREE_P], p[2 * TREE_P], Sr, Sz, Sp);
+        for (int i = turn; i < lne; i += step) add(le0 + i);
+        turn = (turn - lne) & (step - 1);
       }
     }
-    if (nl > TREE_LIST - 32) flush();
+    if (nl > TREE_FLUSH) flush();
     __syncwarp();
   }
   flush();
