@@ -5,7 +5,7 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from test_gpu_tree import _lens
+from test_gpu_tree import _arc, _lens, _points, _polyline, _scale, _sources
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,80 @@ def _some_single():
 def test_single_element_runs_are_shared_by_the_team(cuda, n, tw):
     t = _Trace(cuda, _some_single(), n, tw)
     assert _time(lambda: t.run(True)) <= 1.5 * _time(lambda: t.run(False))
+
+
+def _mesh(kind, n):
+    if kind == 'lens':
+        return _lens(n)
+    if kind == 'cone':
+        return _polyline([(0.5, -2.0), (1.5, -1.0), (2.5, 2.0)], [n // 2, n - n // 2])
+    if kind == 'shuffled':
+        return _lens(n)[np.random.default_rng(0).permutation(n)]
+    if kind == 'mixed':
+        return np.concatenate([_arc(n // 4), _lens(n - n // 4)])
+    return _arc(n)
+
+
+MESHES = ['lens', 'arc', 'cone', 'shuffled', 'mixed']
+
+
+def _both(cuda, pts, src, pot=None):
+    """The field by both entries: what to call, and where it goes."""
+    import torch
+    M, Nq = pts.shape[0], src.shape[1]
+    nbytes = cuda.backend_lib.tb_field_points_workspace(M, Nq)
+    assert nbytes > 0
+    work = cuda.dev_scratch(nbytes, pts.device)
+    f = torch.empty((2, M, 3), dtype=torch.float64, device=pts.device)
+    p = torch.empty((2, M), dtype=torch.float64, device=pts.device)
+    ptr = (lambda i: p[i].data_ptr()) if pot else (lambda i: None)
+    args = pts.data_ptr(), M, src.data_ptr(), Nq
+    return (lambda: cuda._call('tb_field_radial_points_ws', *args, ptr(0), f[0].data_ptr(), work.data_ptr(), nbytes,
+                               cuda._stream()),
+            lambda: cuda._call('tb_field_radial_points', *args, ptr(1), f[1].data_ptr(), cuda._stream()), f, p)
+
+
+@pytest.mark.parametrize('kind', MESHES)
+@pytest.mark.parametrize('M', [64, 512, 4096])
+def test_points_are_not_slower_than_the_direct_sums(cuda, kind, M):
+    import torch
+    rng = np.random.default_rng(M)
+    src = _sources(cuda, _mesh(kind, 4096), rng.uniform(0.5, 2, 4096))
+    pts = cuda.to_dev(np.stack([rng.uniform(0, 2e-3, M), np.zeros(M), rng.uniform(-5e-3, 5e-3, M)], 1), torch.float64)
+    tree, direct, _, _ = _both(cuda, pts, src)
+    # on 64 points the build takes a third of the direct sums' time
+    assert _time(tree) <= 1.5 * _time(direct)
+
+
+@pytest.mark.parametrize('kind', MESHES)
+@pytest.mark.parametrize('M', [64, 74, 75, 148, 149, 296, 297, 592, 593, 1184, 1185])  # 32, 16, 8, 4, 2 and 1 warps a point
+def test_points_with_several_warps(cuda, kind, M):
+    import torch
+    v = _mesh(kind, 4096)
+    rng = np.random.default_rng(M)
+    q = rng.standard_normal(len(v))
+    src = _sources(cuda, v, q)
+    p = _points(rng, v, max(M, 300))[:M]
+    pts = cuda.to_dev(p, torch.float64)
+    tree, direct, f, pot = _both(cuda, pts, src, pot=True)
+    tree()
+    direct()
+    # both sums' terms carry the same error of K, E and G; the proxies 2 10^-16 x 2.7 (the Lebesgue constant of 16
+    # nodes) = 6e-16 of them and the stretches' variation 1e-14 (TREE_JITTER) at most; roundings, 65,536 terms in
+    # parts: some 1e-15.  The radial sum's terms are the larger ones of the form that _scale has.
+    tol = 2e-14 * _scale(p, src.cpu().numpy())
+    d = (f[0] - f[1]).abs().cpu().numpy()
+    assert np.all(np.hypot(d[:, 0], d[:, 1]) <= 1.5 * tol[0]) and np.all(d[:, 2] <= tol[1])
+    assert np.all((pot[0] - pot[1]).abs().cpu().numpy() <= tol[2])
+
+
+@pytest.mark.parametrize('kind', ['arc', 'cone', 'shuffled'])
+@pytest.mark.parametrize('n, tw', [(1, 8), (1024, 4), (4096, 1)])
+def test_traces_are_not_slower_than_the_direct_sums(cuda, kind, n, tw):
+    import torch
+    t = _Trace(cuda, _mesh(kind, 800), n, tw)
+    assert _time(lambda: t.run(True)) <= 1.25 * _time(lambda: t.run(False))
+    t.run(True)
+    plane, count = t.plane.clone(), t.count.clone()
+    t.run(False)
+    assert torch.equal(torch.isfinite(plane), torch.isfinite(t.plane)) and torch.equal(count, t.count)

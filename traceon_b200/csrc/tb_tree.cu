@@ -7,13 +7,15 @@
 //   k_tree_nodes     one warp per node: extent and proxies, first the nodes of
 //                    at most TREE_MID elements from their rings, then, in a
 //                    second launch, the larger ones from these nodes' proxies
-//   k_field_points_tree  one warp per point
+//   k_field_points_tree  1 to 32 warps per point
 //
 // The build reads the rings once and interpolates them log2(TREE_MID /
 // TREE_LEAF) + 1 times; it is latency-bound (four short launches: 24 us for
 // 1,000 elements, 100 us for 16,384).  A point then sums some 400 rings
 // whatever the mesh: 2^18 points on 16,384 elements take 0.9 ms where the
 // direct sums took 410, 9,797 points on 1,537 elements 0.07 ms instead of 1.8.
+#include <cooperative_groups.h>
+
 #include "tb_tree.cuh"
 #include "../../include/traceon_b200.h"
 
@@ -121,8 +123,39 @@ __device__ __forceinline__ int run_slots(int m, int axis) {
   return axis == TREE_DIRECT || l < 2 ? 1 : (1 << (l - 1)) - 1;
 }
 
+// Whether the tree is of use is known here only: every point sums at least one
+// chunk for each straight run and all chunks of the others, and each of a
+// team's eight warps looks at every run (some eighth of a chunk's time).  Where
+// that is more than all elements, each group becomes one run without proxies:
+// its rings in the given order (elements in random order, 800 of them, one
+// electron with eight warps: 2.0 times the direct sums' time through their runs
+// of one element each, 1.1 so).
 __global__ void __launch_bounds__(TR_THREADS) k_tree_runs(Tree T, const int64_t* __restrict__ offsets) {
   __shared__ int sums[32];
+  __shared__ int least;  // those chunks, and the runs
+  if (threadIdx.x == 0) least = 0;
+  __syncthreads();
+  int mine = 0;
+  for (int e = 4 * threadIdx.x; e < T.n; e += 4 * TR_THREADS) {
+    const uchar4 q = *reinterpret_cast<const uchar4*>(T.kind + e);  // the layout rounds kind's bytes up
+    const uint8_t k[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      if (e + i < T.n) mine += ((k[i] & 3) == TREE_DIRECT ? 1 : k[i] >> 2) + (k[i] >> 2);
+  }
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if ((threadIdx.x & 31) == 0) atomicAdd(&least, mine);
+  __syncthreads();
+  if (least > T.n) {
+    for (int e = threadIdx.x; e < T.n; e += TR_THREADS) T.kind[e] = uint8_t(TREE_DIRECT + (e == 0 ? 4 : 0));
+    __syncthreads();
+    if (offsets)
+      for (int g = threadIdx.x; g < T.groups; g += TR_THREADS) {
+        const int64_t e = offsets[g] / TREE_P;
+        if (e >= 0 && e < T.n) T.kind[e] = uint8_t(TREE_DIRECT + 4);
+      }
+    __syncthreads();
+  }
   int runs = 0, total;
   for (int base = 0; base < T.n; base += TR_THREADS) {
     const int e = base + threadIdx.x;
@@ -183,6 +216,7 @@ __device__ __forceinline__ double cheb_x(int m) { return cospi((2 * m + 1) / (2.
 template <bool MID>
 __global__ void __launch_bounds__(128) k_tree_nodes(Tree T) {
   __shared__ double sx[TREE_P], sb[TREE_P];
+  if (blockIdx.x * (int64_t)(blockDim.x / 32) >= T.count[1]) return;
   if (threadIdx.x < TREE_P) {
     sx[threadIdx.x] = cheb_x(threadIdx.x);
     sb[threadIdx.x] = sinpi((2 * threadIdx.x + 1) / (2.0 * TREE_P)) * (threadIdx.x & 1 ? -1.0 : 1.0);
@@ -319,25 +353,84 @@ int tree_build(const Tree& T, const double* src, const int64_t* offsets, cudaStr
   return launch_status();
 }
 
-constexpr int FT_THREADS = 256;
+// PARTS warps per point, 1 to 32: what fills the chip's resident warps, so that
+// few points on a mesh without straight stretches are not left to one warp
+// each (4,096 elements of arcs: 64 points 960 us with one warp a point, 67 with
+// 32, the direct sums 150; 512 points 960, 296 with four, 340).  16 and 32 are
+// a cluster of CTAs.
+constexpr int FT_WARPS = 8;  // of a CTA, two CTAs a SM
 
-template <bool POT>
-__global__ void __launch_bounds__(FT_THREADS, 2)
+template <bool POT, int PARTS>
+__global__ void __launch_bounds__(32 * FT_WARPS, 2)
     k_field_points_tree(Tree T, const double* __restrict__ points, int64_t M, double* __restrict__ pot,
                         double* __restrict__ field) {
-  __shared__ TreeScratch sc[FT_THREADS / 32];
+  namespace cg = cooperative_groups;
+  constexpr int CTAS = PARTS > FT_WARPS ? PARTS / FT_WARPS : 1, PER_CTA = PARTS > FT_WARPS ? 1 : FT_WARPS / PARTS;
+  __shared__ TreeScratch sc[FT_WARPS];
+  __shared__ double red[PARTS > 1 ? FT_WARPS * CTAS : 1][3];
   const int w = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int part = (CTAS > 1 ? FT_WARPS * int(blockIdx.x % CTAS) : 0) + w % (PARTS / CTAS);
   const int runs = T.count[0];
-  for (int64_t m = blockIdx.x * (int64_t)(FT_THREADS / 32) + w; m < M; m += (int64_t)gridDim.x * (FT_THREADS / 32)) {
-    const double p[3] = {points[3 * m], points[3 * m + 1], points[3 * m + 2]};
-    const double r0 = axis_distance(p);
-    double Sr = 0, Sz = 0, Sp = 0;
-    tree_sums<POT>(T, 0, runs, r0, p[2], sc[w], 0, 1, Sr, Sz, Sp);
-    Sr = warp_sum(Sr);
-    Sz = warp_sum(Sz);
-    if (POT) Sp = warp_sum(Sp);
-    if (lane == 0) finish_field(p, Sr, Sz, Sp, pot, field, m);
+  const int point = w * CTAS / PARTS;  // of the CTA's; where warps share one they all stay in the loop together
+  for (int64_t m = blockIdx.x / CTAS * (int64_t)PER_CTA + point; (PARTS > 1 ? m - point : m) < M;
+       m += int64_t(gridDim.x / CTAS) * PER_CTA) {
+    const bool in = PARTS == 1 || m < M;
+    double p[3], Sr = 0, Sz = 0, Sp = 0;
+    if (in) {
+      for (int k = 0; k < 3; k++) p[k] = points[3 * m + k];
+      const double r0 = axis_distance(p);
+      tree_sums<POT>(T, 0, runs, r0, p[2], sc[w], part, PARTS, Sr, Sz, Sp);
+      Sr = warp_sum(Sr);
+      Sz = warp_sum(Sz);
+      if (POT) Sp = warp_sum(Sp);
+    }
+    if (PARTS > 1) {  // the first of the point's warps adds them up
+      if (CTAS > 1) cg::this_cluster().sync();  // the other CTAs run, and the last sums are taken
+      if (lane == 0) {
+        double* to = &red[CTAS > 1 ? part : w][0];
+        if (CTAS > 1) to = cg::this_cluster().map_shared_rank(to, 0);
+        to[0] = Sr;
+        to[1] = Sz;
+        to[2] = Sp;
+      }
+      if (CTAS > 1)
+        cg::this_cluster().sync();
+      else
+        __syncthreads();
+      if (part == 0) {
+        for (int k = 1; k < PARTS; k++) {
+          Sr += red[w + k][0];
+          Sz += red[w + k][1];
+          Sp += red[w + k][2];
+        }
+      }
+      if (CTAS == 1) __syncthreads();
+    }
+    if (in && part == 0 && lane == 0) finish_field(p, Sr, Sz, Sp, pot, field, m);
   }
+}
+
+template <int PARTS>
+static void launch_points_tree(const Tree& T, const double* points, int64_t M, double* pot, double* field,
+                               cudaStream_t s) {
+  constexpr int CTAS = PARTS > FT_WARPS ? PARTS / FT_WARPS : 1;
+  int64_t blocks = (M * PARTS + FT_WARPS - 1) / FT_WARPS;
+  const int64_t resident = (int64_t)num_sms() * 2 / CTAS * CTAS;
+  if (blocks > resident) blocks = resident;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(32 * FT_WARPS);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = CTAS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  if (pot)  // errors: launch_status()
+    cudaLaunchKernelEx(&cfg, k_field_points_tree<true, PARTS>, T, points, M, pot, field);
+  else
+    cudaLaunchKernelEx(&cfg, k_field_points_tree<false, PARTS>, T, points, M, pot, field);
 }
 
 }  // namespace tb
@@ -345,8 +438,10 @@ __global__ void __launch_bounds__(FT_THREADS, 2)
 using namespace tb;
 
 extern "C" int64_t tb_field_points_workspace(int64_t M, int64_t Nq) {
-  // The line between the two: the build's some 25 us against the pairs that it
-  // saves, 1e11 to 2e11 a second (4e6 pairs: 20 to 40 us).
+  // The line between the two: the build's some 40 us (14 where the tree turns
+  // out to be of no use) against the pairs that it saves.  64 points on 4,096
+  // elements, 4.2e6 pairs: 60 us on a lens, 67 on arcs, cones or elements in
+  // random order, 150 by the direct sums; 2,000 points 77, 1,140 and 1,165.
   if (M <= 0 || Nq <= 0 || Nq % TREE_P != 0 || Nq / TREE_P > TREE_MAX_ELEMENTS) return 0;
   if (M < 64 || double(M) * double(Nq) < 4e6) return 0;
   return tree_layout(Nq / TREE_P, 1, nullptr, nullptr);
@@ -364,11 +459,18 @@ extern "C" int tb_field_radial_points_ws(const double* points, int64_t M, const 
   tree_layout(Nq / TREE_P, 1, static_cast<char*>(work), &T);
   const int st = tree_build(T, sources, nullptr, s);
   if (st != OK) return st;
-  int64_t blocks = (M + FT_THREADS / 32 - 1) / (FT_THREADS / 32);
-  if (blocks > (int64_t)num_sms() * 2) blocks = (int64_t)num_sms() * 2;
-  if (pot)
-    k_field_points_tree<true><<<unsigned(blocks), FT_THREADS, 0, s>>>(T, points, M, pot, field);
+  const int64_t warps = (int64_t)num_sms() * 2 * FT_WARPS;  // resident on the chip
+  if (M * 32 <= warps)
+    launch_points_tree<32>(T, points, M, pot, field, s);
+  else if (M * 16 <= warps)
+    launch_points_tree<16>(T, points, M, pot, field, s);
+  else if (M * 8 <= warps)
+    launch_points_tree<8>(T, points, M, pot, field, s);
+  else if (M * 4 <= warps)
+    launch_points_tree<4>(T, points, M, pot, field, s);
+  else if (M * 2 <= warps)
+    launch_points_tree<2>(T, points, M, pot, field, s);
   else
-    k_field_points_tree<false><<<unsigned(blocks), FT_THREADS, 0, s>>>(T, points, M, pot, field);
+    launch_points_tree<1>(T, points, M, pot, field, s);
   return launch_status();
 }
