@@ -504,8 +504,8 @@ int tb_trace_rk45_geometries(const double *start, const double *t0, const double
  * tree_work (16-byte aligned) before it traces.  Fields with magnetostatic or
  * current rings are summed directly.
  * tb_trace_workspace gives the bytes (n_geoms: 0 without geom); where that is
- * 0 or tree_work is NULL, the direct sums run.  With geom the source offsets
- * have to be multiples of 16. */
+ * 0 or tree_work is NULL, the direct sums run, and so they do with geom where
+ * a source offset is not a multiple of 16. */
 int64_t tb_trace_workspace(const tb_field_t *field, int64_t n, int64_t n_geoms);
 int tb_trace_rk45_ws(const double *start, const double *t0, const double *qm, const int32_t *geom, int64_t n,
                      const tb_field_t *field, const int64_t *src_offsets, int64_t n_geoms, const double *geom_bounds,

@@ -147,3 +147,28 @@ def test_traces_are_not_slower_than_the_direct_sums(cuda, kind, n, tw):
     plane, count = t.plane.clone(), t.count.clone()
     t.run(False)
     assert torch.equal(torch.isfinite(plane), torch.isfinite(t.plane)) and torch.equal(count, t.count)
+
+
+@pytest.mark.parametrize('cut', [16 * 150, 16 * 150 + 8, 16 * 150 + 1])
+def test_geometries_that_do_not_start_at_an_element(cuda, cut):
+    """Source offsets that are not multiples of 16 rings: the rings that tb_trace_rk45_geometries sums."""
+    import torch
+    n = 24
+    t = _Trace(cuda, _lens(400), n, 4)
+    geom = torch.arange(n, dtype=torch.int32, device='cuda') % 2
+    off = torch.tensor([0, cut, 16 * 400], dtype=torch.int64, device='cuda')
+    nbytes = cuda.backend_lib.tb_trace_workspace(C.byref(t.field), n, 2)
+    assert nbytes > 0
+    work = cuda.dev_scratch(nbytes, off.device)
+    args = (t.start.data_ptr(), None, t.qm.data_ptr(), geom.data_ptr(), n, C.byref(t.field), off.data_ptr(), 2, None,
+            C.byref(t.o), None, None, t.status.data_ptr(), t.final.data_ptr(), t.plane.data_ptr(), t.count.data_ptr(),
+            t.work.data_ptr())
+    cuda._call('tb_trace_rk45_geometries', *args, cuda._stream())
+    want, count = t.final.clone(), t.count.clone()
+    t.final.zero_()
+    cuda._call('tb_trace_rk45_ws', *args, work.data_ptr(), nbytes, cuda._stream())
+    assert torch.equal(count, t.count)
+    if cut % 16:
+        assert torch.equal(want, t.final)
+    else:  # through the tree; the field differs by some 1e-14, a trace of up to 60 steps by some 1e-12
+        assert bool(((want - t.final).abs() <= 1e-10 * want.abs().amax(0)).all())

@@ -537,6 +537,8 @@ __global__ void __launch_bounds__(TRACE_THREADS, 2) k_trace_bem(TraceParams P) {
   __shared__ double s_red[TEAMS][TW][6];
   __shared__ int64_t s_idx[TEAMS];
   constexpr bool TREE = MODE == BEM_TREE;
+  // geometries with a tree: launched in both modes, and one of them leaves
+  if (GEOM && P.etree.n && (P.etree.count[2] != 0) == TREE) return;
   __shared__ TreeScratch s_tree[TREE ? TRACE_THREADS / 32 : 1];
   const int team = threadIdx.x / T, lt = threadIdx.x % T;
   BemTeamField<TW, GEOM, MODE> field{P, team, lt, s_red[team], &s_tree[TREE ? threadIdx.x / 32 : 0]};
@@ -1644,7 +1646,11 @@ extern "C" int tb_trace_surrogate(const double* start, const double* t0, const d
 template <int TW>
 static int launch_team(const TraceParams& P, bool tree, cudaStream_t s) {
   if (P.nm > 0 || P.nc > 0) return launch_bem<TW, false, BEM_FULL>(P, s);
-  if (P.geom) return tree ? launch_bem<TW, true, BEM_TREE>(P, s) : launch_bem<TW, true, BEM_RINGS>(P, s);
+  if (P.geom) {
+    // whether the offsets, in device memory, allow a tree is known to the build only
+    const int st = tree ? launch_bem<TW, true, BEM_TREE>(P, s) : OK;
+    return st == OK ? launch_bem<TW, true, BEM_RINGS>(P, s) : st;
+  }
   return tree ? launch_bem<TW, false, BEM_TREE>(P, s) : launch_bem<TW, false, BEM_RINGS>(P, s);
 }
 

@@ -52,8 +52,7 @@ __device__ __forceinline__ int rings_axis(double r, double z, double w, double& 
   return TREE_DIRECT;
 }
 
-// offsets (groups + 1), multiples of 16: the first ring of each group; null:
-// one group.
+// offsets (groups + 1): the first ring of each group; null: one group.
 __global__ void __launch_bounds__(256)
     k_tree_elements(Tree T, const double* __restrict__ src, const int64_t* __restrict__ offsets) {
   const int64_t nq = int64_t(T.n) * TREE_P;
@@ -178,10 +177,15 @@ __global__ void __launch_bounds__(TR_THREADS) k_tree_runs(Tree T, const int64_t*
     if (i < runs) T.run_slot[i] = at;
     slots += total;
   }
+  int split = 0;
+  if (offsets)
+    for (int g = threadIdx.x; g <= T.groups; g += TR_THREADS) split |= offsets[g] % TREE_P != 0;
+  split = __syncthreads_or(split);
   if (threadIdx.x == 0) {
     T.run_slot[runs] = slots;
     T.count[0] = runs;
     T.count[1] = slots;
+    T.count[2] = split != 0;
   }
   for (int g = threadIdx.x; g <= T.groups; g += TR_THREADS) {
     const int64_t e = g == T.groups && !offsets ? T.n : (offsets ? offsets[g] / TREE_P : 0);

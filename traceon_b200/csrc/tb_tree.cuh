@@ -71,7 +71,7 @@ struct Tree {
   int* run_e0 = nullptr;     // [runs + 1] first element of each run
   int* run_slot = nullptr;   // [runs + 1] its root's slot
   int* group_run = nullptr;  // [groups + 1] first run of each group of rings
-  int* count = nullptr;      // [2] runs, slots
+  int* count = nullptr;      // [3] runs, slots, whether a group does not start at an element
   int n = 0;                 // elements
   int groups = 0;
 };
@@ -94,7 +94,7 @@ inline int64_t tree_layout(int64_t n, int64_t groups, char* work, Tree* t) {
   x.run_e0 = reinterpret_cast<int*>(take((n + 1) * 4));
   x.run_slot = reinterpret_cast<int*>(take((n + 1) * 4));
   x.group_run = reinterpret_cast<int*>(take((groups + 1) * 4));
-  x.count = reinterpret_cast<int*>(take(8));
+  x.count = reinterpret_cast<int*>(take(3 * 4));
   x.n = int(n);
   x.groups = int(groups);
   if (t) *t = x;
@@ -102,6 +102,9 @@ inline int64_t tree_layout(int64_t n, int64_t groups, char* work, Tree* t) {
 }
 
 // Builds the tree of the rings src (3, 16 n) on the stream (tb_tree.cu).
+// offsets (groups + 1, device memory): the first ring of each group, or null
+// for one group.  Where one is not a multiple of 16 (count[2]) the tree is not
+// that of the groups.
 int tree_build(const Tree& T, const double* src, const int64_t* offsets, cudaStream_t s);
 
 // Scratch of one warp's walk.  A round of the walk takes at most 32 nodes off
