@@ -591,17 +591,25 @@ def to_dev(a, dtype=None):
 def dev_scratch(nbytes, device, stream=None):
     """Device scratch (uint8) for a call on `stream` (a raw stream, default the
     current one), or None for 0 bytes and when memory is short: every call that
-    takes such scratch has a form without."""
+    takes such scratch has a form without.  It comes from that stream's own
+    memory, so it may be dropped as soon as the call is enqueued, and is never a
+    block that work on another stream still uses."""
     torch = _torch()
     if nbytes <= 0:
         return None
+    other = stream is not None and stream != _stream()
     try:
-        t = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device) if other else None):
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
         return None
-    if stream is not None and stream != _stream():  # used there, allocated here
-        t.record_stream(torch.cuda.ExternalStream(stream, device=device))
-    return t
+
+
+def dev_capturing(device, stream):
+    """Whether the raw stream is part of a graph capture."""
+    torch = _torch()
+    with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device)):
+        return torch.cuda.is_current_stream_capturing()
 
 
 def dev_jacobian_buffer(vertices_t):

@@ -151,6 +151,9 @@ class Tracer:
         if r != B.TB_OK:
             raise B.BackendError(f'tb_trace_rk45 failed with status {r}')
         res = TraceResult(status, final, plane, counters, rows, nrows)
+        # the tree's scratch (0.85 KB an element) is the stream's again, unless a graph will write it on each replay
+        if tree is not None and not B.dev_capturing(dev, s):
+            tree = None
         res._keep = (keep, start, qm, t0, work, tree)
         return res
 
