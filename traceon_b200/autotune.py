@@ -22,6 +22,7 @@ The table is the library's only mutable global state; `clear()` empties it.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 import threading
 
@@ -62,15 +63,25 @@ def _time_ms(fn, reps: int = 2) -> float:
     return best
 
 
-def best_team_warps(tracer, start, qm, atol: float, max_attempts: int, rings: int, sample: int = 4096) -> int:
+def sums_kind(field, n: int) -> tuple:
+    """What an evaluation of `field` (a TbField) sums, as the tracer's kernels
+    distinguish it: ('tree' | 'rings' | 'magnetic', its bucket of current rings)."""
+    if field.n_mag > 0 or field.n_cur > 0:
+        return 'magnetic', _bucket(field.n_cur)
+    return ('tree' if B.backend_lib.tb_trace_workspace(C.byref(field), n, 0) > 0 else 'rings'), 0
+
+
+def best_team_warps(tracer, start, qm, atol: float, max_attempts: int, rings: int, sample: int = 4096,
+                    kind: tuple = ()) -> int:
     """Fastest team size of the plain BEM tracer for this field and particle
     count.  The sample keeps the particle count of the real launch up to
     `sample` particles (so occupancy is the same); larger launches are tuned on
     `sample` particles spread over the batch and reuse the choice per size
-    bucket.  `rings`: ring sources summed per field evaluation."""
+    bucket.  `rings`: ring sources summed per field evaluation; `kind`: how
+    (sums_kind: some 400 rings of a tree and all of them want other teams)."""
     torch = B._torch()
     n = start.shape[0]
-    key = ('bem_team_warps', torch.cuda.get_device_name(start.device), _bucket(rings), _bucket(n))
+    key = ('bem_team_warps', torch.cuda.get_device_name(start.device), (_bucket(rings), *kind), _bucket(n))
     with _lock:
         if key in _table:
             return _table[key]
@@ -99,13 +110,13 @@ def tune_batch_pipeline(pipe, sample: int = 4096) -> dict:
     every team size on `sample` of its particles spread over the batch (at
     most 2,000 attempts each); the fastest of each is set on `pipe` (before
     its graph is captured) and kept per device and size bucket (total tiles,
-    rings, particles).  Returns
+    rings, particles, whether the trace has its tree).  Returns
     {'blocks_per_sm': b, 'team_warps': tw, 'times_ms': {...}}."""
     torch = B._torch()
     bs = pipe.batch
     tiles = int(sum(p[0] * p[0] for p in bs.plan))
     key = ('batch_pipeline', torch.cuda.get_device_name(bs.work.device), _bucket(tiles), _bucket(bs.rings),
-           _bucket(pipe.n))
+           _bucket(pipe.n), pipe.tree is not None)
     with _lock:
         hit = _table.get(key)
     if hit is None:

@@ -124,7 +124,8 @@ class Tracer:
             from . import autotune
             team_warps = 0
             if f.axial_z is None and n:
-                team_warps = autotune.best_team_warps(self, start, qm, atol, max_attempts, f.n_elec + f.n_mag)
+                team_warps = autotune.best_team_warps(self, start, qm, atol, max_attempts, f.n_elec + f.n_mag,
+                                                      kind=autotune.sums_kind(f, n))
         o = B.TbTraceOpts()
         for i, v in enumerate(self.bounds.reshape(-1)):
             o.bounds[i] = float(v)
