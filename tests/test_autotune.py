@@ -72,9 +72,6 @@ def test_team_sizes_are_kept_apart_by_what_is_summed(monkeypatch):
     from traceon_b200 import backend as B
     from traceon_b200.tracing import Tracer
 
-    class Stop(Exception):
-        pass
-
     chosen = []
 
     class Lib:

@@ -39,9 +39,10 @@ __device__ __forceinline__ void finish_field(const double* p, double Sr, double 
                                              double* field, int64_t m) {
   if (pot) pot[m] = Sp * INV_PI;
   if (field) {
-    const double er = axis_distance(p) >= MIN_AXIS ? Sr * INV_PI : 0.0;  // E_r / r
-    field[3 * m] = p[0] * er;
-    field[3 * m + 1] = p[1] * er;
+    const bool off_axis = axis_distance(p) >= MIN_AXIS;  // not where a coordinate is no number
+    const double er = Sr * INV_PI;                       // E_r / r
+    field[3 * m] = off_axis ? p[0] * er : 0.0;
+    field[3 * m + 1] = off_axis ? p[1] * er : 0.0;
     field[3 * m + 2] = -Sz * INV_PI;
   }
 }
