@@ -18,11 +18,13 @@ electrodes), the axial series alone (the same table, no network), and the
 plain FP64 BEM tracer on a 16,384-electron slice.  Endpoint errors of the
 surrogate and of the axial series against the CPU oracle on a held-out
 sample of each beam (1 % of the headline beam), traced in spawned processes
-while the GPU works; CPU baselines: the reference C backend's plain-BEM
-tracer and its axial-series tracer on all host threads.
+while the GPU works; CPU baselines: the plain-BEM tracer and the axial-series
+tracer of the reference C backend (where it is built in oracle/_ref, else of
+its restatement in oracle/, `kind` "port") on all host threads.
 
   --field bem: the plain FP64 BEM field only.
-  --impl reference: the reference C backend's plain BEM tracer on host cores.
+  --impl reference: the reference C backend's plain BEM tracer on host cores
+      (oracle/_ref; unavailable where that is not built).
   --workload solve: only the precision workload's solve (the lens at
       --precision-n elements, 8 right-hand sides): GPU FP64 fill, FP64
       pivoted LU and the mixed tensor-core solve (also reported, as
@@ -215,11 +217,15 @@ def endpoint_errors_nm(plane, ref_xy):
             'within_1nm': int(np.sum(d <= 1.0))}
 
 
+CPU_TRACERS = {'ref': 'the reference C backend', 'port': "this repository's C restatement of the reference backend"}
+
+
 def cpu_reference_rate(q, jac, pos, p0, v0, threads, seconds, kind='ref', axial=None):
     """The reference's own CPU tracer (oracle/_ref: trace_particle with its
     field_radial_traceable callback, or with field_radial_derivs_traceable
     when `axial` = (z, coefficients) is given) on `threads` host threads for
-    about `seconds`; returns (electrons/s, electrons traced, kind)."""
+    about `seconds`; where it is not built, the restatement's (kind 'port').
+    Returns (electrons/s, electrons traced, kind)."""
     from oracle.oracle import Oracle, EM, available
     from traceon_b200 import geometry as G
     if kind == 'ref' and not available('ref'):
@@ -256,8 +262,8 @@ def cpu_reference_rate(q, jac, pos, p0, v0, threads, seconds, kind='ref', axial=
 
 def reference_axial_table(q, jac, pos, z):
     """The reference's FieldRadialAxial table of the oracle charges on the
-    grid z: its C axial-derivative sums (oracle/_ref) and its SciPy spline
-    coefficients (traceon/field.py:971-991)."""
+    grid z: its C axial-derivative sums (oracle/_ref, or the restatement's) and
+    its SciPy spline coefficients (traceon/field.py:971-991)."""
     from oracle.oracle import Oracle, available, axial_coefficients
     o = Oracle('ref' if available('ref') else 'port')
     return axial_coefficients(z, o.axial_derivatives_radial(z, q, jac, pos))
@@ -274,6 +280,11 @@ def host_cores():
 def run_reference(args):
     ws, rank, _ = dist_info()
     if rank != 0:
+        return
+    from oracle.oracle import available
+    if not available('ref'):
+        print(json.dumps({'impl': 'reference', 'unavailable': 'the reference C backend (oracle/_ref) is not built: '
+                                                              'its sources are not here'}), flush=True)
         return
     cores = host_cores()
     geo, volts, p0, v0 = lens_inputs(4096, args.beam)
@@ -296,7 +307,7 @@ def run_reference(args):
             'config': workload_config(args.electrons, args.field, args.beam),
             'reference_field': 'plain BEM (the reference has no learned surrogate)',
             'cpu_baseline': {'value': value, 'unit': 'electrons/s', 'cores': cores,
-                             'kind': 'reference' if kind == 'ref' else 'port',
+                             'kind': 'reference',
                              'sample': f'{n_total} electrons of this beam over {args.steps} steps of ~{step_s:.0f} s '
                                        f'(reference C backend trace_particle + field_radial_traceable, '
                                        f'{cores} threads)'},
@@ -411,8 +422,8 @@ def precision_solve(n, nrhs=8, seed=2, field_points=1 << 20, fp64_lu=True, fp64_
 
 def fp64_roofline(units, flop_per_unit, ms, peak, kernel, unit_desc, direct=True):
     """direct=False: the kernel does not compute each unit (ring tree, short Gauss rules), so the rate of the units
-    that it stands for is no fraction of the peak."""
-    achieved = units * flop_per_unit / (ms * 1e-3) / 1e12
+    that it stands for is no rate of arithmetic."""
+    achieved = units * flop_per_unit / (ms * 1e-3) / 1e12 if direct else None
     return {'bound': 'fp64', 'kernel': kernel, 'units': units, 'flop_per_unit': flop_per_unit,
             'unit_desc': unit_desc, 'achieved': achieved, 'unit': 'TFLOP/s', 'peak': peak,
             'frac': achieved / peak if peak and direct else None, 'counts': 'computed' if direct else 'direct-sum units',
@@ -759,8 +770,8 @@ def run_gpu(args):
             row['plain_bem'] = {'value': ws * m / launch_s, 'electrons': m, 'ms_per_step': float(np.mean(ms_b)),
                                 'kernel': 'k_trace_bem',
                                 'roofline': {'bound': 'fp64', 'unit': 'TFLOP/s', 'flop_per_pair': FLOP_FIELD_PAIR,
-                                             'achieved': pairs * FLOP_FIELD_PAIR / launch_s / 1e12,
-                                             'counts': 'direct-sum units', 'frac': None,
+                                             'units': pairs, 'achieved': None, 'counts': 'direct-sum units',
+                                             'frac': None,
                                              'unit_desc': 'ring-pair field evaluations of the direct sums, which the '
                                                           'tracer takes through its ring tree'}}
             row['speedup_surrogate_vs_plain_bem'] = row['surrogate']['value'] / row['plain_bem']['value']
@@ -805,8 +816,7 @@ def run_gpu(args):
             rf['peak_source'] = 'FP64 FMA throughput measured in this run (tests/probe tb_probe_fp64_fma)'
     else:
         pairs_per_launch = attempts * 6 * Nq
-        achieved = pairs_per_launch * FLOP_FIELD_PAIR / launch_s / 1e12
-        roof = {'bound': 'fp64', 'achieved': achieved, 'peak': fp64_peak, 'unit': 'TFLOP/s',
+        roof = {'bound': 'fp64', 'achieved': None, 'peak': fp64_peak, 'unit': 'TFLOP/s',
                 'frac': None, 'counts': 'direct-sum units', 'traffic': None, 'kernel': 'k_trace_bem',
                 'flop_per_unit': FLOP_FIELD_PAIR, 'units_per_launch': pairs_per_launch,
                 'unit_desc': 'ring-pair field evaluations of the direct sums, which the tracer takes through its ring '
@@ -847,13 +857,13 @@ def run_gpu(args):
     elif precision is not None:
         precision.pop('_field_state', None)
 
-    # ---- CPU baselines (rank 0, N = 1): the reference's plain-BEM tracer and
-    # its axial-series tracer on this beam, all host threads, bounded samples
+    # ---- CPU baselines (rank 0, N = 1): the reference's (or the restatement's) plain-BEM
+    # tracer and axial-series tracer on this beam, all host threads, bounded samples
     cpu = cpu_axial = None
     if ws == 1 and args.cpu_seconds > 0 and q_or is not None:
         rate, n, kind = cpu_reference_rate(q_or, jac_or, pos_or, p0, v0, cores, args.cpu_seconds)
         cpu = {'value': rate, 'unit': 'electrons/s', 'cores': cores, 'kind': 'reference' if kind == 'ref' else 'port',
-               'sample': f'{n} electrons of this beam traced by the reference C backend (trace_particle + '
+               'sample': f'{n} electrons of this beam traced by {CPU_TRACERS[kind]} (trace_particle + '
                          f'field_radial_traceable, plain BEM; the reference has no surrogate) on {cores} threads '
                          f'for ~{args.cpu_seconds:.0f} s'}
         if sur is not None:
@@ -862,7 +872,7 @@ def run_gpu(args):
                                                axial=(sur.z, coeffs))
             cpu_axial = {'value': rate, 'unit': 'electrons/s', 'cores': cores,
                          'kind': 'reference' if kind == 'ref' else 'port',
-                         'sample': f'{n} electrons of this beam traced by the reference C backend through its axial '
+                         'sample': f'{n} electrons of this beam traced by {CPU_TRACERS[kind]} through its axial '
                                    f'series (trace_particle + field_radial_derivs_traceable, FieldRadialAxial '
                                    f'table of {len(sur.z)} z-points) on {cores} threads for '
                                    f'~{args.cpu_seconds / 2:.0f} s'}
@@ -1239,7 +1249,8 @@ def run_batch(args):
                                                      float(np.percentile(counters[:, 1], 99)),
                                                      int(counters[:, 1].max())]},
             'trace_roofline': fp64_roofline(pairs, FLOP_FIELD_PAIR, trace_ms, fp64_peak, 'k_trace_bem',
-                                            'ring-pair field evaluations (+ 1 log, 1 rsqrt, 1 reciprocal each)'),
+                                            'ring-pair field evaluations (+ 1 log, 1 rsqrt each); through the ring tree '
+                                            'where the pipeline has one', direct=pipe.tree is None),
             'setup_s': setup_s, 'accuracy': acc, 'clocks': clk.summary()}
     print(json.dumps(line), flush=True)
 
