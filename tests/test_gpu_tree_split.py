@@ -149,6 +149,19 @@ def test_traces_are_not_slower_than_the_direct_sums(cuda, kind, n, tw):
     assert torch.equal(torch.isfinite(plane), torch.isfinite(t.plane)) and torch.equal(count, t.count)
 
 
+@pytest.mark.parametrize('kind', MESHES)
+@pytest.mark.parametrize('n, tw', [(3, 8), (70, 1)])
+def test_traces_are_ring_by_ring_where_the_tree_is_of_no_use(cuda, kind, n, tw):
+    """... bit for bit, and through the tree otherwise."""
+    import torch
+    t = _Trace(cuda, _mesh(kind, 400), n, tw)
+    t.run(True)
+    final, count = t.final.clone(), t.count.clone()
+    t.run(False)
+    same = torch.equal(final, t.final)
+    assert torch.equal(count, t.count) and same == (kind in ('arc', 'cone', 'shuffled'))
+
+
 @pytest.mark.parametrize('cut', [16 * 150, 16 * 150 + 8, 16 * 150 + 1])
 def test_geometries_that_do_not_start_at_an_element(cuda, cut):
     """Source offsets that are not multiples of 16 rings: the rings that tb_trace_rk45_geometries sums."""

@@ -597,9 +597,10 @@ def dev_scratch(nbytes, device, stream=None):
     torch = _torch()
     if nbytes <= 0:
         return None
-    other = stream is not None and stream != _stream()
     try:
-        with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device) if other else None):
+        if stream is None or stream == _stream():
+            return torch.empty(nbytes, dtype=torch.uint8, device=device)
+        with torch.cuda.stream(torch.cuda.ExternalStream(stream, device=device)):
             return torch.empty(nbytes, dtype=torch.uint8, device=device)
     except torch.OutOfMemoryError:
         return None

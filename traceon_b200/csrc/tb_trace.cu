@@ -254,8 +254,8 @@ __device__ __forceinline__ void team_barrier(int team, int nthreads) {
 }
 
 // How a team sums its rings.  Through the tree (tb_tree.cuh) 4,096 electrons
-// in the field of 1,000 elements take 7.3 ms, ring by ring 190 ms; a sweep of
-// eight lenses with 128 electrons each 3.3 ms instead of 73.
+// in the field of 1,000 elements take 8.0 ms, ring by ring 190 ms; a sweep of
+// eight lenses with 128 electrons each 2.9 ms instead of 73.
 enum BemMode : int {
   BEM_RINGS = 0,  // electrostatic rings, one by one
   BEM_TREE = 1,   // electrostatic rings through their tree
@@ -272,7 +272,11 @@ enum BemMode : int {
 // step on, and that step's error estimate (1e-14 m, from positions of 1e-4 m)
 // consists of the sums' last bits; through the step length these show in the
 // final state at 1e-9 of it, so any other form or order of the sums, however
-// exact, ends there.
+// exact, ends elsewhere by that much (measured with the other form: 1.3e-9 to
+// 1.9e-9 of one electron's end state, for which this form is kept).  It is the
+// less exact one near the axis: E_r and H_r are off by 1.4e-11 at 0.1 mm and
+// 5.5e-9 at 1 um from it (the forces there vanish with r), and differ by that
+// from the field that the point sums give.
 template <int TW, bool GEOM, int MODE>
 struct BemTeamField {
   const TraceParams& P;
@@ -537,8 +541,8 @@ __global__ void __launch_bounds__(TRACE_THREADS, 2) k_trace_bem(TraceParams P) {
   __shared__ double s_red[TEAMS][TW][6];
   __shared__ int64_t s_idx[TEAMS];
   constexpr bool TREE = MODE == BEM_TREE;
-  // geometries with a tree: launched in both modes, and one of them leaves
-  if (GEOM && P.etree.n && (P.etree.count[2] != 0) == TREE) return;
+  // with a tree: launched in both modes, and one of them leaves
+  if (MODE != BEM_FULL && P.etree.n && (P.etree.count[2] != 0) == TREE) return;
   __shared__ TreeScratch s_tree[TREE ? TRACE_THREADS / 32 : 1];
   const int team = threadIdx.x / T, lt = threadIdx.x % T;
   BemTeamField<TW, GEOM, MODE> field{P, team, lt, s_red[team], &s_tree[TREE ? threadIdx.x / 32 : 0]};
@@ -1646,12 +1650,13 @@ extern "C" int tb_trace_surrogate(const double* start, const double* t0, const d
 template <int TW>
 static int launch_team(const TraceParams& P, bool tree, cudaStream_t s) {
   if (P.nm > 0 || P.nc > 0) return launch_bem<TW, false, BEM_FULL>(P, s);
-  if (P.geom) {
-    // whether the offsets, in device memory, allow a tree is known to the build only
-    const int st = tree ? launch_bem<TW, true, BEM_TREE>(P, s) : OK;
-    return st == OK ? launch_bem<TW, true, BEM_RINGS>(P, s) : st;
+  // Whether the tree is of use, and the offsets (in device memory) allow it, only
+  // its build knows: both kernels are launched and one leaves at once (3 us).
+  if (tree) {
+    const int st = P.geom ? launch_bem<TW, true, BEM_TREE>(P, s) : launch_bem<TW, false, BEM_TREE>(P, s);
+    if (st != OK) return st;
   }
-  return tree ? launch_bem<TW, false, BEM_TREE>(P, s) : launch_bem<TW, false, BEM_RINGS>(P, s);
+  return P.geom ? launch_bem<TW, true, BEM_RINGS>(P, s) : launch_bem<TW, false, BEM_RINGS>(P, s);
 }
 
 static int trace_rk45(const double* start, const double* t0, const double* qm, const int32_t* geom, int64_t n,

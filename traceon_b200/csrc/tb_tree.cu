@@ -11,9 +11,10 @@
 //
 // The build reads the rings once and interpolates them log2(TREE_MID /
 // TREE_LEAF) + 1 times; it is latency-bound (four short launches: 24 us for
-// 1,000 elements, 100 us for 16,384).  A point then sums some 400 rings
-// whatever the mesh: 2^18 points on 16,384 elements take 0.9 ms where the
-// direct sums took 410, 9,797 points on 1,537 elements 0.07 ms instead of 1.8.
+// 1,000 elements, 100 us for 16,384).  A point near straight stretches then
+// sums some 400 rings however many there are: 2^18 points on 16,384 elements
+// of a lens take 0.9 ms where the direct sums took 410, 9,797 points on 1,537
+// elements 0.08 ms instead of 1.8.
 #include <cooperative_groups.h>
 
 #include "tb_tree.cuh"
@@ -128,24 +129,30 @@ __device__ __forceinline__ int run_slots(int m, int axis) {
 // that is more than all elements, each group becomes one run without proxies:
 // its rings in the given order (elements in random order, 800 of them, one
 // electron with eight warps: 2.0 times the direct sums' time through their runs
-// of one element each, 1.1 so).
+// of one element each, 1.1 so; the tracer sums ring by ring then).
 __global__ void __launch_bounds__(TR_THREADS) k_tree_runs(Tree T, const int64_t* __restrict__ offsets) {
   __shared__ int sums[32];
-  __shared__ int least;  // those chunks, and the runs
+  __shared__ int least;  // those chunks
   if (threadIdx.x == 0) least = 0;
-  __syncthreads();
-  int mine = 0;
-  for (int e = 4 * threadIdx.x; e < T.n; e += 4 * TR_THREADS) {
-    const uchar4 q = *reinterpret_cast<const uchar4*>(T.kind + e);  // the layout rounds kind's bytes up
-    const uint8_t k[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      if (e + i < T.n) mine += ((k[i] & 3) == TREE_DIRECT ? 1 : k[i] >> 2) + (k[i] >> 2);
-  }
-  mine = __reduce_add_sync(0xffffffffu, mine);
-  if ((threadIdx.x & 31) == 0) atomicAdd(&least, mine);
-  __syncthreads();
-  if (least > T.n) {
+  int runs, total;
+  bool useless = false;
+  for (;;) {
+    runs = 0;
+    int mine = 0;
+    for (int base = 0; base < T.n; base += TR_THREADS) {
+      const int e = base + threadIdx.x;
+      const int k = e < T.n ? T.kind[e] : TREE_HORIZONTAL, s = k >> 2;
+      mine += (k & 3) == TREE_DIRECT ? 1 : s;
+      const int at = runs + cta_scan(s, sums, total);
+      if (s) T.run_e0[at] = e;
+      runs += total;
+    }
+    if (useless) break;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (mine && (threadIdx.x & 31) == 0) atomicAdd(&least, mine);
+    __syncthreads();
+    useless = least + runs > T.n;
+    if (!useless) break;
     for (int e = threadIdx.x; e < T.n; e += TR_THREADS) T.kind[e] = uint8_t(TREE_DIRECT + (e == 0 ? 4 : 0));
     __syncthreads();
     if (offsets)
@@ -154,14 +161,6 @@ __global__ void __launch_bounds__(TR_THREADS) k_tree_runs(Tree T, const int64_t*
         if (e >= 0 && e < T.n) T.kind[e] = uint8_t(TREE_DIRECT + 4);
       }
     __syncthreads();
-  }
-  int runs = 0, total;
-  for (int base = 0; base < T.n; base += TR_THREADS) {
-    const int e = base + threadIdx.x;
-    const int s = e < T.n && (T.kind[e] & 4) ? 1 : 0;
-    const int at = runs + cta_scan(s, sums, total);
-    if (s) T.run_e0[at] = e;
-    runs += total;
   }
   if (threadIdx.x == 0) T.run_e0[runs] = T.n;
   __syncthreads();
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_tree_runs(Tree T, const int64_t*
     T.run_slot[runs] = slots;
     T.count[0] = runs;
     T.count[1] = slots;
-    T.count[2] = split != 0;
+    T.count[2] = split != 0 || useless;
   }
   for (int g = threadIdx.x; g <= T.groups; g += TR_THREADS) {
     const int64_t e = g == T.groups && !offsets ? T.n : (offsets ? offsets[g] / TREE_P : 0);
@@ -421,16 +420,24 @@ static void launch_points_tree(const Tree& T, const double* points, int64_t M, d
   int64_t blocks = (M * PARTS + FT_WARPS - 1) / FT_WARPS;
   const int64_t resident = (int64_t)num_sms() * 2 / CTAS * CTAS;
   if (blocks > resident) blocks = resident;
+  const unsigned threads = 32 * FT_WARPS;
+  if (CTAS == 1) {
+    if (pot)
+      k_field_points_tree<true, PARTS><<<unsigned(blocks), threads, 0, s>>>(T, points, M, pot, field);
+    else
+      k_field_points_tree<false, PARTS><<<unsigned(blocks), threads, 0, s>>>(T, points, M, pot, field);
+    return;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(blocks));
-  cfg.blockDim = dim3(32 * FT_WARPS);
+  cfg.blockDim = dim3(threads);
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = CTAS;
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = CTAS > 1 ? 1 : 0;
+  cfg.numAttrs = 1;
   if (pot)  // errors: launch_status()
     cudaLaunchKernelEx(&cfg, k_field_points_tree<true, PARTS>, T, points, M, pot, field);
   else

@@ -71,7 +71,7 @@ struct Tree {
   int* run_e0 = nullptr;     // [runs + 1] first element of each run
   int* run_slot = nullptr;   // [runs + 1] its root's slot
   int* group_run = nullptr;  // [groups + 1] first run of each group of rings
-  int* count = nullptr;      // [3] runs, slots, whether a group does not start at an element
+  int* count = nullptr;      // [3] runs, slots, 1: of no use, or a group does not start at an element
   int n = 0;                 // elements
   int groups = 0;
 };
@@ -103,8 +103,8 @@ inline int64_t tree_layout(int64_t n, int64_t groups, char* work, Tree* t) {
 
 // Builds the tree of the rings src (3, 16 n) on the stream (tb_tree.cu).
 // offsets (groups + 1, device memory): the first ring of each group, or null
-// for one group.  Where one is not a multiple of 16 (count[2]) the tree is not
-// that of the groups.
+// for one group.  Where one is not a multiple of 16 (count[2] is 1 then) the tree
+// is not that of the groups.
 int tree_build(const Tree& T, const double* src, const int64_t* offsets, cudaStream_t s);
 
 // Scratch of one warp's walk.  A round of the walk takes at most 32 nodes off
