@@ -1236,8 +1236,10 @@ def run_batch(args):
                                    f'+-50 mrad), direct BEM field, RKF45 atol {args.batch_atol:g} m',
                        'geometries': ng, 'electrons_per_geometry': ne, 'elements_total': int(Ns.sum()),
                        'elements_min_max': [int(Ns.min()), int(Ns.max())]},
-            'graph': {'launches_per_replay': 2, 'kernels': ['k_batch_solve', 'k_trace_bem'],
-                      'memset_nodes_per_replay': 3},
+            'graph': {'launches_per_replay': 2 if pipe.tree is None else 7,
+                      'kernels': ['k_batch_solve'] + ([] if pipe.tree is None else
+                                                      ['k_tree_elements', 'k_tree_runs', 'k_tree_nodes']) +
+                      ['k_trace_bem'], 'memset_nodes_per_replay': 3},
             'solve_ms': float(np.mean(solve_ms)), 'trace_ms': trace_ms,
             'solve_status': {'ok': int(np.sum(status_solve == 0)), 'fallback_lu': int(np.sum(status_solve == 5))},
             'autotune': tuned,
@@ -1302,8 +1304,8 @@ def main():
     ap.add_argument('--ref-seconds', type=float, default=20.0)
     # DRAM bytes (read + write) of one full-size launch of the dominant kernel
     # from an ncu capture of this workload (k_trace_surrogate_tc, wide beam:
-    # 17.06 MB read + 2.80 MB written; see the profile summary of that kernel)
-    ap.add_argument('--traffic', type=float, default=19.86e6)
+    # 16.89 MB read + 1.90 MB written; see the profile summary of that kernel)
+    ap.add_argument('--traffic', type=float, default=18.80e6)
     args = ap.parse_args()
     if args.impl == 'reference':
         run_reference(args)

@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(256)
 
 // One cluster of CTAs (1, 2, 4 or 8) per point, for a few points: a CTA alone
 // would leave the other SMs idle for as long as its 256 threads take (one
-// point on 16,000 rings: 35 us with one CTA, 6 with eight).  Each CTA's sums
+// point on 16,000 rings: 35 us with one CTA, 8.5 with eight).  Each CTA's sums
 // go to the first one's shared memory and are added there in a fixed order.
 constexpr int FP_CLUSTER = 8;
 template <bool POT>
