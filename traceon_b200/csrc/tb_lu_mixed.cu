@@ -1270,7 +1270,10 @@ static SideStream g_side[64][SIDE_SLOTS];
 static unsigned long long capture_of(cudaStream_t s) {
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
-  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) return 0;
+  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) {
+    cudaGetLastError();  // not an error of a launch: those on s report their own
+    return 0;
+  }
   if (status == cudaStreamCaptureStatusInvalidated) return ~0ull;
   return status == cudaStreamCaptureStatusActive ? id : 0;
 }
